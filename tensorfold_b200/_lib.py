@@ -1,4 +1,5 @@
-"""ctypes binding of ``libtensorfold_b200.so`` (the C ABI in ``include/tensorfold_b200.h``).
+"""Binding of ``libtensorfold_b200.so`` (the C ABI in ``include/tensorfold_b200.h``): the native functions of
+``csrc/host.cpp``, and the same entry points through ctypes.
 
 There is no fallback: if the library is missing, importing a kernel wrapper raises. Tensors cross
 the boundary as raw device pointers; the stream is torch's current stream.
@@ -14,6 +15,7 @@ import torch
 
 HERE = Path(__file__).resolve().parent
 LIB_PATH = HERE / "libtensorfold_b200.so"
+HOST_PATH = HERE / "_host.so"
 
 TF_OK, TF_EINVAL, TF_EALIGN, TF_ESCRATCH, TF_ECUDA, TF_ESTALL = 0, -1, -2, -3, -4, -5
 _NAMES = {TF_EINVAL: "TF_EINVAL (unsupported shape, size or flag)", TF_EALIGN: "TF_EALIGN (misaligned pointer)",
@@ -111,51 +113,48 @@ SIGNATURES: dict[str, tuple] = {
 }
 
 _lib = None
-_launches = 0          # kernel-launching entry points called so far (what a CUDA graph of a step holds)
-_NO_LAUNCH = {"tf_version", "tf_qmm_set_trace", "tf_qmm_tc_set_trace", "tf_set_poll_limit", "tf_qmm_workers", "tf_qmm_scratch_bytes", "tf_packed_bytes", "tf_qmm_tiled_bytes",
-              "tf_attention_scratch_bytes", "tf_attention_chunks", "tf_packed_tc_bytes", "tf_qmm_tc_tiled_bytes", "tf_topk_scratch_bytes", "tf_moe_max_problems", "tf_moe_slot_bytes", "tf_peer_slot_bytes"}
+_host = None
 
 
 def launch_count() -> int:
-    return _launches
+    """Kernels queued by successful calls so far (what a CUDA graph of a step holds)."""
+
+    load()
+    return _host.launch_count()
 
 
-class _Counted:
-    """A bound entry point that counts successful kernel launches (the paged attention and the top-k queue two each)."""
-
-    def __init__(self, fn, n):
-        self.fn, self.n = fn, n
-
-    def __call__(self, *args):
-        global _launches
-        rc = self.fn(*args)
-        if rc == 0:
-            _launches += self.n
-        return rc
+class Bound:
+    """The entry points as attributes: native functions that take the C arguments in order, a pointer being a CUDA
+    tensor, an address or None (``csrc/host.cpp``); ``cdll`` is the same library through ctypes."""
 
 
-
-def load() -> ctypes.CDLL:
+def load():
     """The kernel library, loaded once. Raises if it has not been built."""
 
-    global _lib
+    global _lib, _host
     if _lib is None:
-        if not LIB_PATH.exists():
-            raise RuntimeError(f"{LIB_PATH} is missing: run `python -m tensorfold_b200.build` "
+        if not LIB_PATH.exists() or not HOST_PATH.exists():
+            raise RuntimeError(f"{LIB_PATH} or {HOST_PATH} is missing: run `python -m tensorfold_b200.build` "
                                "(there is no CPU or PyTorch fallback for the lane kernels)")
-        lib = ctypes.CDLL(str(LIB_PATH))
-        class Bound:
-            pass
-
         bound = Bound()
+        bound.cdll = ctypes.CDLL(str(LIB_PATH))
+        from . import _host as host
+
         for name, (res, args) in SIGNATURES.items():
-            fn = getattr(lib, name)
+            fn = getattr(bound.cdll, name)
             fn.restype = res
             fn.argtypes = args
-            setattr(bound, name, fn if name in _NO_LAUNCH else _Counted(fn, 2 if name.startswith("tf_lane_attention_paged") or name == "tf_topk_rows" else 1))
-        bound.cdll = lib
-        _lib = bound
+            setattr(bound, name, getattr(host, name))
+        _host, _lib = host, bound
     return _lib
+
+
+def host():
+    """The native host path (``csrc/host.cpp``): whole operator calls in one native function."""
+
+    if _host is None:
+        load()
+    return _host
 
 
 def check(code: int, what: str) -> None:
@@ -169,7 +168,28 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream (no torch.cuda.Stream object: those took 3 us a call)."""
+
+    return host().current_stream()
+
+
+class _Here:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_here = _Here()
+
+
+def on(device):
+    """Context in which ``device`` is current; nothing to do, and nothing done, where it is already."""
+
+    if device.index is None or device.index == host().current_device():
+        return _here
+    return torch.cuda.device(device)
 
 
 def need_cuda(*tensors: torch.Tensor) -> None:
@@ -195,7 +215,8 @@ _status: dict[int, Status] = {}
 
 
 def status(device) -> Status:
-    idx = torch.device(device).index or 0
-    if idx not in _status:
-        _status[idx] = Status(device)
-    return _status[idx]
+    idx = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    st = _status.get(idx)
+    if st is None:
+        st = _status[idx] = Status(device)
+    return st

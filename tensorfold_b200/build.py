@@ -2,8 +2,8 @@
 
 ``python -m tensorfold_b200.build`` compiles every ``csrc/*.cu`` with nvcc into
 ``tensorfold_b200/libtensorfold_b200.so`` next to this file. The library is plain C ABI
-(``include/tensorfold_b200.h``); Python reaches it through ctypes, so no torch headers are involved
-and the build needs only nvcc.
+(``include/tensorfold_b200.h``) and needs only nvcc; ``csrc/host.cpp``, the native Python binding that takes
+torch tensors, is compiled with g++ into ``_host.so`` beside it and linked against it.
 """
 
 from __future__ import annotations
@@ -19,8 +19,10 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "libtensorfold_b200.so"
+HOST = HERE / "_host.so"
 OBJ = HERE / "build"
 STAMP = OBJ / "sources.sha256"
+HOST_STAMP = OBJ / "host.sha256"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -46,7 +48,37 @@ def source_hash() -> str:
     return h.hexdigest()
 
 
+def _build_host(force: bool) -> None:
+    """``csrc/host.cpp`` -> ``_host.so``: rebuilt when it, the C header or the torch it is compiled against changed."""
+
+    import sysconfig
+
+    import torch
+
+    src, header = CSRC / "host.cpp", HERE.parent / "include" / "tensorfold_b200.h"
+    digest = hashlib.sha256(src.read_bytes() + header.read_bytes() + torch.__version__.encode()).hexdigest()
+    if not force and HOST.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text().strip() == digest:
+        return
+    t = Path(torch.__file__).parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include", str(src),
+           "-o", str(HOST), f"-L{HERE}", "-ltensorfold_b200", f"-L{t}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+           "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed on host.cpp")
+    HOST_STAMP.write_text(digest + "\n")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
+    _build_kernels(force, verbose)
+    _build_host(force)
+    return LIB
+
+
+def _build_kernels(force: bool, verbose: bool) -> Path:
     digest = source_hash()
     if not force and LIB.exists() and STAMP.exists() and STAMP.read_text().strip() == digest:
         return LIB

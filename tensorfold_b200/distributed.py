@@ -122,8 +122,8 @@ class RankGroup:
     def peer_args(self):
         """(buffer pointer table, slot bytes, exchange-number word, ticket word, this rank's buffer) for the fused form."""
 
-        return (self.handle.buffer_ptrs_dev, self.slot_bytes, self.state[0:1].data_ptr(), self.state[1:2].data_ptr(),
-                self.buf.data_ptr())
+        return (self.handle.buffer_ptrs_dev, self.slot_bytes, self.state[0:1], self.state[1:2],
+                self.buf)
 
     def gather_partials(self, local: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """(M, D) fp32 -> (world, M, D) fp32, rank order."""
@@ -141,10 +141,10 @@ class RankGroup:
             local = local.contiguous()
             if out is None:
                 out = torch.empty((self.world, m, d), dtype=torch.float32, device=local.device)
-            with torch.cuda.device(local.device):
-                _lib.check(lib.tf_peer_exchange(local.data_ptr(), m, d, self.handle.buffer_ptrs_dev, self.slot_bytes, out.data_ptr(), self.rank,
-                                                self.world, self.state[0:1].data_ptr(), self.state[1:2].data_ptr(),
-                                                _lib.status(local.device).word.data_ptr(), _lib.stream()), "peer exchange")
+            with _lib.on(local.device):
+                _lib.check(lib.tf_peer_exchange(local, m, d, self.handle.buffer_ptrs_dev, self.slot_bytes, out, self.rank,
+                                                self.world, self.state[0:1], self.state[1:2],
+                                                _lib.status(local.device).word, _lib.stream()), "peer exchange")
             return out
         if out is None:
             out = torch.empty((self.world, *local.shape), dtype=torch.float32, device=local.device)

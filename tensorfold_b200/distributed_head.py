@@ -51,10 +51,10 @@ def choose_split(logits: torch.Tensor, positions: torch.Tensor, sampling, tp, lo
         return midx[:, 0].contiguous()
     rows = midx.shape[0]
     tokens = torch.empty(rows, dtype=torch.int32, device=midx.device)
-    with torch.cuda.device(midx.device):
-        _lib.check(_lib.load().tf_sample_rows(midx.data_ptr(), mval.data_ptr(), k, positions.data_ptr(),
+    with _lib.on(midx.device):
+        _lib.check(_lib.load().tf_sample_rows(midx, mval, k, positions,
                                               int(sampling.seed) & 0xFFFFFFFFFFFFFFFF, float(sampling.temperature),
-                                              int(sampling.top_k), float(sampling.top_p), tokens.data_ptr(), rows,
+                                              int(sampling.top_k), float(sampling.top_p), tokens, rows,
                                               _lib.stream()), "sample_rows")
     return tokens
 

@@ -47,9 +47,9 @@ def choose_rows(values, ids, positions: Sequence[int], s: Sampling) -> list[int]
     pos = torch.as_tensor(list(positions), dtype=torch.int64).to(dev)
     tokens = torch.empty(rows, dtype=torch.int32, device=dev)
     k = max(1, min(int(s.top_k) if s.top_k else width, width))
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().tf_sample_rows(idx.data_ptr(), val.data_ptr(), width, pos.data_ptr(), int(s.seed) & 0xFFFFFFFFFFFFFFFF,
-                                              max(float(s.temperature), 1e-6), k, float(s.top_p), tokens.data_ptr(), rows,
+    with _lib.on(dev):
+        _lib.check(_lib.load().tf_sample_rows(idx, val, width, pos, int(s.seed) & 0xFFFFFFFFFFFFFFFF,
+                                              max(float(s.temperature), 1e-6), k, float(s.top_p), tokens, rows,
                                               _lib.stream()), "choose_rows")
     return [int(t) for t in tokens.cpu()]
 
@@ -81,10 +81,10 @@ def sample_rows(logits: torch.Tensor, positions, s: Sampling | None, *, top: tup
     if positions.shape != (rows,):
         raise ValueError("sample_rows: one position per row")
     tokens = torch.empty(rows, dtype=torch.int32, device=logits.device)
-    with torch.cuda.device(logits.device):
-        _lib.check(_lib.load().tf_sample_rows(idx.data_ptr(), val.data_ptr(), idx.shape[1], positions.data_ptr(),
+    with _lib.on(logits.device):
+        _lib.check(_lib.load().tf_sample_rows(idx, val, idx.shape[1], positions,
                                               int(s.seed) & 0xFFFFFFFFFFFFFFFF, float(s.temperature), int(s.top_k),
-                                              float(s.top_p), tokens.data_ptr(), rows, _lib.stream()), "sample_rows")
+                                              float(s.top_p), tokens, rows, _lib.stream()), "sample_rows")
     return tokens
 
 

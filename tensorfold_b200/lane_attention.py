@@ -103,14 +103,14 @@ def lane_attention(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tensor, k_
         raise ValueError("gate must be the (R, H * 2 * D) bf16 rows of the q projection")
     if packed_out is not None and (packed_out.m != r or packed_out.k != h * d):
         raise ValueError("packed_out must hold R rows of H * D inputs")
-    with torch.cuda.device(q.device):
+    with _lib.on(q.device):
         _lib.check(_lib.load().tf_lane_attention_paged_gated(
-            q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), page_table.data_ptr(),
-            page_table.shape[1], seq_lens.data_ptr(), seq_start.data_ptr(), row_nkeys.data_ptr(), _lib.ptr(out),
-            _lib.ptr(gate), gate.stride(0) if gate is not None else 0,
-            packed_out.data.data_ptr() if packed_out is not None else None, packed_out.group if packed_out is not None else 64,
-            scratch.data_ptr(), scratch.numel(), r, s, max_window, max_chunks, h, hk, d, float(scale),
-            _lib.status(q.device).word.data_ptr(), _lib.stream()), "lane_attention")
+            q, k_new, v_new, k_pages, v_pages, page_table,
+            page_table.shape[1], seq_lens, seq_start, row_nkeys, out,
+            gate, gate.stride(0) if gate is not None else 0,
+            packed_out.data if packed_out is not None else None, packed_out.group if packed_out is not None else 64,
+            scratch, scratch.numel(), r, s, max_window, max_chunks, h, hk, d, float(scale),
+            _lib.status(q.device).word, _lib.stream()), "lane_attention")
     return out if out is not None else packed_out
 
 
@@ -157,10 +157,10 @@ def kv_commit(k_new: torch.Tensor, v_new: torch.Tensor, kv: PagedKV, seq_lens: t
     for all layers at once: k_new, v_new (Layers, R, HK, D)."""
 
     layers, r, hk, d = k_new.shape
-    with torch.cuda.device(k_new.device):
-        _lib.check(_lib.load().tf_kv_commit(k_new.data_ptr(), v_new.data_ptr(), r * hk * d, kv.k.data_ptr(), kv.v.data_ptr(),
-                                            kv.k.stride(0), kv.table.data_ptr(), kv.max_pages, seq_lens.data_ptr(),
-                                            seq_start.data_ptr(), keep.data_ptr(), kv.n_seqs, layers, hk, d, _lib.stream()),
+    with _lib.on(k_new.device):
+        _lib.check(_lib.load().tf_kv_commit(k_new, v_new, r * hk * d, kv.k, kv.v,
+                                            kv.k.stride(0), kv.table, kv.max_pages, seq_lens,
+                                            seq_start, keep, kv.n_seqs, layers, hk, d, _lib.stream()),
                    "kv_commit")
 
 

@@ -49,9 +49,9 @@ def gated_delta_chain(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torc
             raise ValueError("gated_delta_chain: tensors must be contiguous")
     if out is None:
         out = torch.empty((r, hv, dv), dtype=torch.bfloat16, device=q.device)
-    with torch.cuda.device(q.device):
-        _lib.check(_lib.load().tf_gdn_chain(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-                                            state.data_ptr(), _lib.ptr(state_out), out.data_ptr(), seq_start.data_ptr(),
+    with _lib.on(q.device):
+        _lib.check(_lib.load().tf_gdn_chain(q, k, v, g, beta,
+                                            state, state_out, out, seq_start,
                                             s, hk, hv, dk, dv, _lib.stream()), "gated_delta_chain")
     return out
 
@@ -85,12 +85,12 @@ def gdn_mixer(qkv: torch.Tensor, z: torch.Tensor, a: torch.Tensor, b: torch.Tens
             raise ValueError("gdn_mixer: state, weights and record tensors must be contiguous")
     packed = out if out is not None else new_packed(r, nv * 128, group, qkv.device)
     rows = torch.empty((r, nv * 128), dtype=torch.bfloat16, device=qkv.device) if rows_out else None
-    with torch.cuda.device(qkv.device):
+    with _lib.on(qkv.device):
         _lib.check(_lib.load().tf_gdn_fused(
-            qkv.data_ptr(), qkv.stride(0), z.data_ptr(), z.stride(0), a.data_ptr(), b.data_ptr(), a.stride(0),
-            conv_state.data_ptr(), conv_weight.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), norm_weight.data_ptr(),
-            state.data_ptr(), k_rec.data_ptr(), v_rec.data_ptr(), g_rec.data_ptr(), beta_rec.data_ptr(), packed.data.data_ptr(),
-            _lib.ptr(rows), seq_start.data_ptr(), r, s, nk, nv, 128, 128, 4, group, float(eps), _lib.stream()), "gdn_mixer")
+            qkv, qkv.stride(0), z, z.stride(0), a, b, a.stride(0),
+            conv_state, conv_weight, a_log, dt_bias, norm_weight,
+            state, k_rec, v_rec, g_rec, beta_rec, packed.data,
+            rows, seq_start, r, s, nk, nv, 128, 128, 4, group, float(eps), _lib.stream()), "gdn_mixer")
     return (packed, rows) if rows_out else packed
 
 
@@ -145,9 +145,9 @@ def replay(k: torch.Tensor, v: torch.Tensor, g: torch.Tensor, beta: torch.Tensor
     for t in (k, v, g, beta, state):
         if not t.is_contiguous():
             raise ValueError("replay: tensors must be contiguous")
-    with torch.cuda.device(k.device):
-        _lib.check(_lib.load().tf_gdn_replay(k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(), state.data_ptr(),
-                                             seq_start.data_ptr(), keep.data_ptr(), s, layers, r * hk * dk, r * hv * dv,
+    with _lib.on(k.device):
+        _lib.check(_lib.load().tf_gdn_replay(k, v, g, beta, state,
+                                             seq_start, keep, s, layers, r * hk * dk, r * hv * dv,
                                              r * hv, s * hv * dv * dk, hk, hv, dk, dv, _lib.stream()), "replay")
 
 
@@ -161,10 +161,10 @@ def conv_commit(qkv: torch.Tensor, conv_state: torch.Tensor, seq_start: torch.Te
     many = qkv.dim() == 3
     layers = qkv.shape[0] if many else 1
     s = conv_state.shape[-3]
-    with torch.cuda.device(qkv.device):
-        _lib.check(_lib.load().tf_conv_commit(qkv.data_ptr(), qkv.stride(-2), qkv.stride(0) if many else 0,
-                                              conv_state.data_ptr(), conv_state.stride(0) if many else 0,
-                                              seq_start.data_ptr(), keep.data_ptr(), s, layers, channels, _lib.stream()),
+    with _lib.on(qkv.device):
+        _lib.check(_lib.load().tf_conv_commit(qkv, qkv.stride(-2), qkv.stride(0) if many else 0,
+                                              conv_state, conv_state.stride(0) if many else 0,
+                                              seq_start, keep, s, layers, channels, _lib.stream()),
                    "conv_commit")
 
 

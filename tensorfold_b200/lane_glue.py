@@ -64,16 +64,16 @@ def norm_xs(hidden: torch.Tensor, residual: torch.Tensor | None, weight: torch.T
     h = h_out if has_res else hidden
     packed = (out if out is not None else new_packed(m, d, group, hidden.device)) if packed_out else None
     rows = torch.empty_like(hidden) if rows_out else None
-    with torch.cuda.device(hidden.device):
+    with _lib.on(hidden.device):
         if peer is not None:
             _, slot_bytes, seq, tickets, mine = peer.peer_args()
         else:
             slot_bytes, seq, tickets, mine = 0, None, None, None
-        _lib.check(_lib.load().tf_norm_xs_peer(hidden.data_ptr(), _lib.ptr(residual), _lib.ptr(partials), nparts, pstride,
-                                               weight.data_ptr(), _lib.ptr(h_out) if has_res else None, _lib.ptr(rows),
-                                               packed.data.data_ptr() if packed else None, m, d, group, float(eps),
+        _lib.check(_lib.load().tf_norm_xs_peer(hidden, residual, partials, nparts, pstride,
+                                               weight, h_out if has_res else None, rows,
+                                               packed.data if packed else None, m, d, group, float(eps),
                                                mine, slot_bytes, seq, tickets, peer.world if peer is not None else 0,
-                                               _lib.status(hidden.device).word.data_ptr(), _lib.stream()), "norm_xs")
+                                               _lib.status(hidden.device).word, _lib.stream()), "norm_xs")
     if packed_out and rows_out:
         return h, packed, rows
     return h, (packed if packed_out else rows)
@@ -91,9 +91,9 @@ def mlp_act(gate: torch.Tensor, up: torch.Tensor, *, group: int = 64, rows_out: 
         raise ValueError("mlp_act: gate and up must be (M, I) views with the same row stride")
     packed = out if out is not None else new_packed(m, n, group, gate.device)
     rows = torch.empty((m, n), dtype=torch.bfloat16, device=gate.device) if rows_out else None
-    with torch.cuda.device(gate.device):
-        _lib.check(_lib.load().tf_swiglu(gate.data_ptr(), up.data_ptr(), gate.stride(0), packed.data.data_ptr(),
-                                         _lib.ptr(rows), m, n, group, _lib.stream()), "mlp_act")
+    with _lib.on(gate.device):
+        _lib.check(_lib.load().tf_swiglu(gate, up, gate.stride(0), packed.data,
+                                         rows, m, n, group, _lib.stream()), "mlp_act")
     return (packed, rows) if rows_out else packed
 
 
@@ -112,8 +112,8 @@ def mlp_act_tiled(gate_up: torch.Tensor, intermediate: int, *, group: int = 64, 
         raise ValueError("mlp_act_tiled: gate_up must be (M, >= 2 I) rows")
     packed = out if out is not None else new_packed(m, intermediate, group, gate_up.device)
     rows = torch.empty((m, intermediate), dtype=torch.bfloat16, device=gate_up.device) if rows_out else None
-    with torch.cuda.device(gate_up.device):
-        _lib.check(_lib.load().tf_swiglu_tiled(gate_up.data_ptr(), gate_up.stride(0), packed.data.data_ptr(), _lib.ptr(rows), m,
+    with _lib.on(gate_up.device):
+        _lib.check(_lib.load().tf_swiglu_tiled(gate_up, gate_up.stride(0), packed.data, rows, m,
                                                intermediate, group, _lib.stream()), "mlp_act_tiled")
     return (packed, rows) if rows_out else packed
 
@@ -131,9 +131,9 @@ def gdn_post(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps: float,
     y = y.contiguous()
     packed = out if out is not None else new_packed(m, nv * dv, group, y.device)
     rows = torch.empty((m, nv * dv), dtype=torch.bfloat16, device=y.device) if rows_out else None
-    with torch.cuda.device(y.device):
-        _lib.check(_lib.load().tf_gated_norm(y.data_ptr(), z.data_ptr(), z.stride(0), weight.data_ptr(),
-                                             packed.data.data_ptr(), _lib.ptr(rows), m, nv, dv, group, float(eps),
+    with _lib.on(y.device):
+        _lib.check(_lib.load().tf_gated_norm(y, z, z.stride(0), weight,
+                                             packed.data, rows, m, nv, dv, group, float(eps),
                                              _lib.stream()), "gdn_post")
     return (packed, rows) if rows_out else packed
 
@@ -153,9 +153,9 @@ def gate_mul(o: torch.Tensor, qg: torch.Tensor, *, heads: int, head_dim: int, gr
     o = o.contiguous()
     packed = out if out is not None else new_packed(m, heads * head_dim, group, o.device)
     rows = torch.empty((m, heads * head_dim), dtype=torch.bfloat16, device=o.device) if rows_out else None
-    with torch.cuda.device(o.device):
-        _lib.check(_lib.load().tf_gate_mul(o.data_ptr(), qg.data_ptr(), qg.stride(0), packed.data.data_ptr(),
-                                           _lib.ptr(rows), m, heads, head_dim, group, _lib.stream()), "gate_mul")
+    with _lib.on(o.device):
+        _lib.check(_lib.load().tf_gate_mul(o, qg, qg.stride(0), packed.data,
+                                           rows, m, heads, head_dim, group, _lib.stream()), "gate_mul")
     return (packed, rows) if rows_out else packed
 
 
@@ -178,11 +178,11 @@ def attn_prep(qg: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_norm: torch.
                torch.empty((m, kv_heads, head_dim), dtype=torch.bfloat16, device=dev),
                torch.empty((m, kv_heads, head_dim), dtype=torch.bfloat16, device=dev))
     qo, ko, vo = out
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().tf_attn_prep(qg.data_ptr(), qg.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(),
-                                            v.stride(0), q_norm.data_ptr(), k_norm.data_ptr(), pos.data_ptr(),
-                                            inv_freq.data_ptr(), inv_freq.numel(), qo.data_ptr(), ko.data_ptr(),
-                                            vo.data_ptr(), m, heads, kv_heads, head_dim, float(eps), _lib.stream()),
+    with _lib.on(dev):
+        _lib.check(_lib.load().tf_attn_prep(qg, qg.stride(0), k, k.stride(0), v,
+                                            v.stride(0), q_norm, k_norm, pos,
+                                            inv_freq, inv_freq.numel(), qo, ko,
+                                            vo, m, heads, kv_heads, head_dim, float(eps), _lib.stream()),
                    "attn_prep")
     return qo, ko, vo
 
@@ -209,11 +209,11 @@ def gdn_pre(qkv: torch.Tensor, conv_state: torch.Tensor, conv_weight: torch.Tens
                torch.empty((m, nv, dv), dtype=torch.bfloat16, device=dev), torch.empty((m, nv), dtype=torch.float32, device=dev),
                torch.empty((m, nv), dtype=torch.float32, device=dev))
     q, k, v, g, beta = out
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().tf_gdn_pre(qkv.data_ptr(), qkv.stride(0), conv_state.data_ptr(), conv_weight.data_ptr(),
-                                          row_seq.data_ptr(), row_idx.data_ptr(), a.data_ptr(), b.data_ptr(), a.stride(0),
-                                          a_log.data_ptr(), dt_bias.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                          g.data_ptr(), beta.data_ptr(), m, nk, nv, dk, dv, 4, _lib.stream()), "gdn_pre")
+    with _lib.on(dev):
+        _lib.check(_lib.load().tf_gdn_pre(qkv, qkv.stride(0), conv_state, conv_weight,
+                                          row_seq, row_idx, a, b, a.stride(0),
+                                          a_log, dt_bias, q, k, v,
+                                          g, beta, m, nk, nv, dk, dv, 4, _lib.stream()), "gdn_pre")
     return q, k, v, g, beta
 
 
@@ -227,9 +227,9 @@ def embed(ids: torch.Tensor, weight: torch.Tensor, scales: torch.Tensor, biases:
     m = ids.shape[0]
     if out is None:
         out = torch.empty((m, d), dtype=torch.bfloat16, device=ids.device)
-    with torch.cuda.device(ids.device):
-        _lib.check(_lib.load().tf_embed(ids.data_ptr(), weight.data_ptr(), scales.data_ptr(), biases.data_ptr(),
-                                        out.data_ptr(), m, d, group, weight.shape[0], _lib.stream()), "embed")
+    with _lib.on(ids.device):
+        _lib.check(_lib.load().tf_embed(ids, weight, scales, biases,
+                                        out, m, d, group, weight.shape[0], _lib.stream()), "embed")
     return out
 
 

@@ -132,8 +132,8 @@ def router(x: torch.Tensor, router_rows: torch.Tensor, out: torch.Tensor | None 
     ne = router_rows.shape[0]
     if out is None:
         out = torch.empty((m, ne), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.load().tf_moe_router(x.data_ptr(), x.stride(0), router_rows.contiguous().data_ptr(), out.data_ptr(), m, d, ne,
+    with _lib.on(x.device):
+        _lib.check(_lib.load().tf_moe_router(x, x.stride(0), router_rows.contiguous(), out, m, d, ne,
                                              _lib.stream()), "moe router")
     return out
 
@@ -144,13 +144,13 @@ def select(logits: torch.Tensor, buf: MoEBuffers, ep: ExpertGroup | None = None)
 
     lib = _lib.load()
     rows = logits.shape[0]
-    with torch.cuda.device(logits.device):
-        _lib.check(lib.tf_moe_select(logits.data_ptr(), rows, buf.total, buf.experts, buf.top_k, buf.pick.data_ptr(),
-                                     buf.wts.data_ptr(), _lib.stream()), "moe select")
-        _lib.check(lib.tf_moe_group(buf.pick.data_ptr(), rows, buf.slots, buf.total, buf.max_probs, buf.prob_expert.data_ptr(),
-                                    buf.prob_count.data_ptr(), buf.prob_rows.data_ptr(), buf.pair_loc.data_ptr(), buf.experts,
-                                    ep.rank if ep else 0, ep.world if ep else 1, buf.prob_sel.data_ptr() if ep else None,
-                                    buf.sel_count.data_ptr() if ep else None, _lib.stream()), "moe group")
+    with _lib.on(logits.device):
+        _lib.check(lib.tf_moe_select(logits, rows, buf.total, buf.experts, buf.top_k, buf.pick,
+                                     buf.wts, _lib.stream()), "moe select")
+        _lib.check(lib.tf_moe_group(buf.pick, rows, buf.slots, buf.total, buf.max_probs, buf.prob_expert,
+                                    buf.prob_count, buf.prob_rows, buf.pair_loc, buf.experts,
+                                    ep.rank if ep else 0, ep.world if ep else 1, buf.prob_sel if ep else None,
+                                    buf.sel_count if ep else None, _lib.stream()), "moe group")
 
 
 def moe(x: torch.Tensor, router_rows: torch.Tensor, ex: Experts, buf: MoEBuffers, ep: ExpertGroup | None = None) -> torch.Tensor:
@@ -169,35 +169,35 @@ def moe(x: torch.Tensor, router_rows: torch.Tensor, ex: Experts, buf: MoEBuffers
     router(x, router_rows, buf.logits)
     select(buf.logits, buf, ep)
     count = buf.sel_count if ep else buf.prob_count
-    sel = buf.prob_sel.data_ptr() if ep else None
+    sel = buf.prob_sel if ep else None
     scratch = scratch_for(dev)
     st = _lib.status(dev)
     g, inter = buf.group, buf.intermediate
-    with torch.cuda.device(dev):
+    with _lib.on(dev):
         s = _lib.stream()
-        _lib.check(lib.tf_moe_pack(x.data_ptr(), x.stride(0), buf.prob_rows.data_ptr(), buf.prob_count.data_ptr(), buf.max_probs,
-                                   buf.x_packed.data_ptr(), d, g, s), "moe pack")
-        _lib.check(lib.tf_qmm_grouped(buf.x_packed.data_ptr(), ex.gate_up.data_ptr(), buf.prob_expert.data_ptr(),
-                                      count.data_ptr(), sel, buf.max_probs, buf.gate_up.data_ptr(), scratch.data_ptr(),
-                                      scratch.numel(), 2 * inter, d, g, 0, st.word.data_ptr(), s), "moe gate_up")
-        _lib.check(lib.tf_moe_act(buf.gate_up.data_ptr(), buf.prob_count.data_ptr(), buf.max_probs, buf.act_packed.data_ptr(), inter,
+        _lib.check(lib.tf_moe_pack(x, x.stride(0), buf.prob_rows, buf.prob_count, buf.max_probs,
+                                   buf.x_packed, d, g, s), "moe pack")
+        _lib.check(lib.tf_qmm_grouped(buf.x_packed, ex.gate_up, buf.prob_expert,
+                                      count, sel, buf.max_probs, buf.gate_up, scratch,
+                                      scratch.numel(), 2 * inter, d, g, 0, st.word, s), "moe gate_up")
+        _lib.check(lib.tf_moe_act(buf.gate_up, buf.prob_count, buf.max_probs, buf.act_packed, inter,
                                   g, s), "moe act")
-        _lib.check(lib.tf_qmm_grouped(buf.act_packed.data_ptr(), ex.down.data_ptr(), buf.prob_expert.data_ptr(),
-                                      count.data_ptr(), sel, buf.max_probs, buf.y.data_ptr(), scratch.data_ptr(),
-                                      scratch.numel(), d, inter, g, 1, st.word.data_ptr(), s), "moe down")
+        _lib.check(lib.tf_qmm_grouped(buf.act_packed, ex.down, buf.prob_expert,
+                                      count, sel, buf.max_probs, buf.y, scratch,
+                                      scratch.numel(), d, inter, g, 1, st.word, s), "moe down")
         if ep is None:
-            _lib.check(lib.tf_moe_combine(buf.y.data_ptr(), buf.pair_loc.data_ptr(), buf.wts.data_ptr(), buf.slots,
-                                          buf.out.data_ptr(), rows, d, s), "moe combine")
+            _lib.check(lib.tf_moe_combine(buf.y, buf.pair_loc, buf.wts, buf.slots,
+                                          buf.out, rows, d, s), "moe combine")
         else:
             if lib.tf_moe_slot_bytes(buf.max_probs, d) > ep.slot_bytes:
                 raise ValueError("moe: the expert group's exchange buffer is too small for these buffers")
             ep.count += 1
-            _lib.check(lib.tf_moe_push(buf.y.data_ptr(), buf.prob_sel.data_ptr(), buf.sel_count.data_ptr(), buf.max_probs, d,
-                                       ep.handle.buffer_ptrs_dev, ep.slot_bytes, ep.rank, ep.world, ep.state[0:1].data_ptr(), s),
+            _lib.check(lib.tf_moe_push(buf.y, buf.prob_sel, buf.sel_count, buf.max_probs, d,
+                                       ep.handle.buffer_ptrs_dev, ep.slot_bytes, ep.rank, ep.world, ep.state[0:1], s),
                        "moe push")
-            _lib.check(lib.tf_moe_combine_peer(ep.buf.data_ptr(), ep.slot_bytes, buf.pair_loc.data_ptr(), buf.wts.data_ptr(),
-                                               buf.slots, buf.out.data_ptr(), rows, d, ep.world, ep.state[0:1].data_ptr(),
-                                               ep.state[1:2].data_ptr(), st.word.data_ptr(), s), "moe combine (peer)")
+            _lib.check(lib.tf_moe_combine_peer(ep.buf, ep.slot_bytes, buf.pair_loc, buf.wts,
+                                               buf.slots, buf.out, rows, d, ep.world, ep.state[0:1],
+                                               ep.state[1:2], st.word, s), "moe combine (peer)")
     return buf.out
 
 

@@ -64,9 +64,9 @@ def tile_weight(weight: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor
     _lib.need_cuda(weight, scales, biases)
     lib = _lib.load()
     out = torch.empty(lib.tf_qmm_tiled_bytes(n, k, group), dtype=torch.uint8, device=weight.device)
-    with torch.cuda.device(weight.device):
-        _lib.check(lib.tf_qmm_tile(weight.contiguous().data_ptr(), scales.contiguous().data_ptr(),
-                                   biases.contiguous().data_ptr(), out.data_ptr(), n, k, group, _lib.stream()),
+    with _lib.on(weight.device):
+        _lib.check(lib.tf_qmm_tile(weight.contiguous(), scales.contiguous(),
+                                   biases.contiguous(), out, n, k, group, _lib.stream()),
                    "tile_weight")
     return QWeight(out, n, k, group)
 
@@ -79,8 +79,8 @@ def untile_weight(q: QWeight) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]
     words = torch.empty((q.n, q.k // 8), dtype=torch.int32, device=dev)
     scales = torch.empty((q.n, q.k // q.group), dtype=torch.bfloat16, device=dev)
     biases = torch.empty_like(scales)
-    with torch.cuda.device(dev):
-        _lib.check(lib.tf_qmm_untile(q.tiled.data_ptr(), words.data_ptr(), scales.data_ptr(), biases.data_ptr(),
+    with _lib.on(dev):
+        _lib.check(lib.tf_qmm_untile(q.tiled, words, scales, biases,
                                      q.n, q.k, q.group, _lib.stream()), "untile_weight")
     return words, scales, biases
 
@@ -161,8 +161,8 @@ def pack_rows(x: torch.Tensor, group: int = 64, *, want_sums: bool = False):
     x = x.contiguous()
     out = new_packed(m, k, group, x.device)
     xs = torch.empty((m, k // group), dtype=torch.float32, device=x.device) if want_sums else None
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.load().tf_pack_rows(x.data_ptr(), out.data.data_ptr(), _lib.ptr(xs), m, k, group,
+    with _lib.on(x.device):
+        _lib.check(_lib.load().tf_pack_rows(x, out.data, xs, m, k, group,
                                             _lib.stream()), "pack_rows")
     return (out, xs) if want_sums else out
 
@@ -173,18 +173,10 @@ def group_sums(x: torch.Tensor, group: int = 64) -> torch.Tensor:
     return pack_rows(x, group, want_sums=True)[1]
 
 
-_scratch: dict[tuple[int, int], torch.Tensor] = {}
-
-
 def scratch_for(device: torch.device) -> torch.Tensor:
     """Per (device, stream) matmul scratch (zeroed once): parked K segments, their ready tags, launch numbers."""
 
-    key = (device.index or 0, torch.cuda.current_stream(device).cuda_stream)
-    buf = _scratch.get(key)
-    if buf is None:
-        buf = torch.zeros(_lib.load().tf_qmm_scratch_bytes(), dtype=torch.uint8, device=device)
-        _scratch[key] = buf
-    return buf
+    return _lib.host().scratch(device.index or 0)
 
 
 _tiled_cache: dict[tuple, QWeight] = {}
@@ -230,68 +222,49 @@ def lane_matmul(x: torch.Tensor | Packed, weight, scales: torch.Tensor | None = 
         weight = _as_qweight(weight, scales, biases)
     if sk is not None and sk != split_k(weight.n, weight.k):
         raise ValueError(f"lane_matmul: the K schedule is fixed by the shape (split_k = {split_k(weight.n, weight.k)}), got sk={sk}")
-    if isinstance(x, Packed):
-        if x.k != weight.k or x.group != weight.group:
-            raise ValueError(f"lane_matmul: packed rows (K={x.k}, group {x.group}) do not match the weight "
-                             f"(K={weight.k}, group {weight.group})")
-        if x.m > MAX_ROWS:
-            raise ValueError(f"lane_matmul: packed input holds {x.m} rows, at most {MAX_ROWS} per call")
-        chunks, lead, m, dev = [x], (x.m,), x.m, x.data.device
-    else:
-        if x.dtype != torch.bfloat16:
-            raise ValueError("lane_matmul: x must be bf16")
+    nw = next_weight
+    hint = (nw.tiled, nw.n, nw.k, nw.group) if nw is not None else (None, 0, 0, 0)
+    if not isinstance(x, Packed):
+        if peer is None and act_out is None:
+            # plain rows: checks, allocations, packing and launches in one native call
+            return _lib.host().lane_matmul(x, weight.tiled, weight.n, weight.k, weight.group, f32, out, *hint,
+                                           _lib.status(x.device).word if x.is_cuda else None)
         if x.shape[-1] != weight.k:
             raise ValueError(f"lane_matmul: weight (N={weight.n}, K={weight.k}) does not match K={x.shape[-1]}")
-        _lib.need_cuda(x)
-        lead, dev = x.shape[:-1], x.device
-        x2 = x.reshape(-1, weight.k)
-        m = x2.shape[0]
-        if m < 1:
-            raise ValueError("lane_matmul: needs at least one row")
-        chunks = [pack_rows(x2[r0:r0 + MAX_ROWS], weight.group) for r0 in range(0, m, MAX_ROWS)]
+        x = x.reshape(-1, weight.k)
+        if x.shape[0] > MAX_ROWS:
+            raise ValueError(f"lane_matmul: a tensor-parallel partial or a fused SwiGLU is at most {MAX_ROWS} rows")
+        x = pack_rows(x, weight.group)
+    if x.k != weight.k or x.group != weight.group:
+        raise ValueError(f"lane_matmul: packed rows (K={x.k}, group {x.group}) do not match the weight "
+                         f"(K={weight.k}, group {weight.group})")
+    m, dev = x.m, x.data.device
+    if m > MAX_ROWS:
+        raise ValueError(f"lane_matmul: packed input holds {m} rows, at most {MAX_ROWS} per call")
+    scratch = scratch_for(dev)
+    word = _lib.status(dev).word
     if peer is not None:
-        if len(chunks) != 1:
-            raise ValueError("lane_matmul: a tensor-parallel partial is at most MAX_ROWS rows")
         bufs, slot_bytes, seq, _, _ = peer.peer_args()
-        nw = next_weight
-        with torch.cuda.device(dev):
-            scratch = scratch_for(dev)
-            _lib.check(lib.tf_qmm_peer(chunks[0].data.data_ptr(), weight.tiled.data_ptr(), scratch.data_ptr(), scratch.numel(), m,
-                                       weight.n, weight.k, weight.group, bufs, slot_bytes, seq, peer.rank, peer.world,
-                                       nw.tiled.data_ptr() if nw is not None else None, nw.n if nw is not None else 0,
-                                       nw.k if nw is not None else 0, nw.group if nw is not None else 0,
-                                       _lib.status(dev).word.data_ptr(), _lib.stream()), "lane_matmul (peer)")
+        with _lib.on(dev):
+            _lib.check(lib.tf_qmm_peer(x.data, weight.tiled, scratch, scratch.numel(), m, weight.n, weight.k, weight.group, bufs, slot_bytes,
+                                       seq, peer.rank, peer.world, *hint, word, _lib.stream()), "lane_matmul (peer)")
         return None
     if act_out is not None:
-        if len(chunks) != 1 or m > 8 or weight.n % 32 or act_out.m != m or act_out.k != weight.n // 2 or act_out.group != weight.group:
+        if m > 8 or weight.n % 32 or act_out.m != m or act_out.k != weight.n // 2 or act_out.group != weight.group:
             raise ValueError("lane_matmul: act_out needs at most 8 rows and a packed buffer of N / 2 inputs")
-        nw = next_weight
-        with torch.cuda.device(dev):
-            scratch = scratch_for(dev)
-            _lib.check(lib.tf_qmm_act(chunks[0].data.data_ptr(), weight.tiled.data_ptr(), act_out.data.data_ptr(), scratch.data_ptr(),
-                                      scratch.numel(), m, weight.n, weight.k, weight.group,
-                                      nw.tiled.data_ptr() if nw is not None else None, nw.n if nw is not None else 0,
-                                      nw.k if nw is not None else 0, nw.group if nw is not None else 0,
-                                      _lib.status(dev).word.data_ptr(), _lib.stream()), "lane_matmul (act)")
+        with _lib.on(dev):
+            _lib.check(lib.tf_qmm_act(x.data, weight.tiled, act_out.data, scratch, scratch.numel(), m, weight.n, weight.k, weight.group,
+                                      *hint, word, _lib.stream()), "lane_matmul (act)")
         return act_out
     dtype = torch.float32 if f32 else torch.bfloat16
     if out is None:
         out = torch.empty((m, weight.n), dtype=dtype, device=dev)
     elif out.shape != (m, weight.n) or out.dtype != dtype or not out.is_contiguous():
         raise ValueError("lane_matmul: out has the wrong shape or dtype")
-    scratch = scratch_for(dev)
-    st = _lib.status(dev)
-    with torch.cuda.device(dev):
-        r0 = 0
-        for c in chunks:
-            nw = next_weight if c is chunks[-1] else weight
-            _lib.check(lib.tf_qmm_next(c.data.data_ptr(), weight.tiled.data_ptr(), out[r0:r0 + c.m].data_ptr(),
-                                       scratch.data_ptr(), scratch.numel(), c.m, weight.n, weight.k, weight.group,
-                                       1 if f32 else 0, nw.tiled.data_ptr() if nw is not None else None,
-                                       nw.n if nw is not None else 0, nw.k if nw is not None else 0,
-                                       nw.group if nw is not None else 0, st.word.data_ptr(), _lib.stream()), "lane_matmul")
-            r0 += c.m
-    return out.reshape(*lead, weight.n)
+    with _lib.on(dev):
+        _lib.check(lib.tf_qmm_next(x.data, weight.tiled, out, scratch, scratch.numel(), m, weight.n, weight.k, weight.group,
+                                   1 if f32 else 0, *hint, word, _lib.stream()), "lane_matmul")
+    return out
 
 
 __all__ = ["MAX_ROWS", "Packed", "QWeight", "group_sums", "lane_matmul", "new_packed", "pack_rows", "pack_scales",

@@ -33,9 +33,9 @@ def topk_rows(x: torch.Tensor, k: int, scratch: torch.Tensor | None = None) -> t
     need = lib.tf_topk_scratch_bytes(rows, vocab, k)
     if scratch is None or scratch.numel() * scratch.element_size() < need:
         scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
-    with torch.cuda.device(x.device):
-        _lib.check(lib.tf_topk_rows(x2.data_ptr(), x2.stride(0), rows, vocab, k, idx.data_ptr(), val.data_ptr(),
-                                    scratch.data_ptr(), scratch.numel() * scratch.element_size(), _lib.stream()), "topk_rows")
+    with _lib.on(x.device):
+        _lib.check(lib.tf_topk_rows(x2, x2.stride(0), rows, vocab, k, idx, val,
+                                    scratch, scratch.numel() * scratch.element_size(), _lib.stream()), "topk_rows")
     return idx, val
 
 
