@@ -420,6 +420,11 @@ size_t tf_topk_scratch_bytes(int rows, int vocab, int k);
 int tf_topk_rows(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, void* scratch,
                  size_t scratch_bytes, void* stream);
 
+/* tf_topk_rows and tf_sample_rows in two launches: each row's token drawn from its k largest logits, which are not written. */
+int tf_topk_sample_rows(const void* x, size_t row_stride, int rows, int vocab, int k, const long long* positions,
+                        unsigned long long seed, double temperature, int top_k, double top_p, int* tokens, void* scratch,
+                        size_t scratch_bytes, void* stream);
+
 /* token = argmax over the kept candidates of val/temperature + Gumbel(splitmix64(seed, position, id));
  * candidates (already ordered as tf_topk_rows writes them) are cut to top_k, then to the smallest
  * prefix whose tempered probability reaches top_p. fp64 arithmetic.

@@ -108,6 +108,8 @@ SIGNATURES: dict[str, tuple] = {
     "tf_set_poll_limit": (None, [ctypes.c_uint]),
     "tf_topk_scratch_bytes": (c_size_t, [c_int, c_int, c_int]),
     "tf_topk_rows": (c_int, [c_void_p, c_size_t, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
+    "tf_topk_sample_rows": (c_int, [c_void_p, c_size_t, c_int, c_int, c_int, c_void_p, c_ulonglong, c_double, c_int, c_double, c_void_p,
+                                    c_void_p, c_size_t, c_void_p]),
     "tf_sample_rows": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_ulonglong, c_double, c_int, c_double, c_void_p,
                                c_int, c_void_p]),
 }

@@ -266,7 +266,7 @@ PyMethodDef methods[] = {
     TF_FN(tf_moe_router, 1), TF_FN(tf_moe_select, 1), TF_FN(tf_moe_group, 1), TF_FN(tf_moe_slot_bytes, 0), TF_FN(tf_moe_push, 1),
     TF_FN(tf_moe_combine_peer, 1), TF_FN(tf_moe_pack, 1), TF_FN(tf_moe_act, 1), TF_FN(tf_moe_combine, 1), TF_FN(tf_peer_slot_bytes, 0),
     TF_FN(tf_peer_exchange, 1), TF_FN(tf_qmm_act, 1), TF_FN(tf_swiglu_tiled, 1), TF_FN(tf_qmm_peer, 1), TF_FN(tf_norm_xs_peer, 1),
-    TF_FN(tf_set_poll_limit, 0), TF_FN(tf_topk_scratch_bytes, 0), TF_FN(tf_topk_rows, 2), TF_FN(tf_sample_rows, 1),
+    TF_FN(tf_set_poll_limit, 0), TF_FN(tf_topk_scratch_bytes, 0), TF_FN(tf_topk_rows, 2), TF_FN(tf_topk_sample_rows, 2), TF_FN(tf_sample_rows, 1),
     TF_OWN("scratch", scratch_py), TF_OWN("lane_matmul", lane_matmul_py), TF_OWN("prefill_matmul", prefill_matmul_py),
     TF_OWN("current_stream", stream_py), TF_OWN("current_device", device_py), TF_OWN("launch_count", count_py),
     {nullptr, nullptr, 0, nullptr}};

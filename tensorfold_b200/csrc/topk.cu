@@ -1,17 +1,23 @@
 // Exact top-k over vocabulary rows and the keyed Gumbel-max draw.
 //
-// top-k: a bf16 logit is a 16-bit sortable key. A row is cut into contiguous slices of at most 16384
-// entries, one CTA per (slice, row). The CTA stages its slice's keys in shared memory, finds the k-th
-// largest key T with two 256-bin histograms (high byte, then low byte), and keeps everything above T
-// plus the ties at T with the SMALLEST token ids: each thread scans a contiguous piece and a
-// block-wide prefix sum places its finds, so no atomic decides which tie survives. A second kernel
-// ranks the slices' candidates by (value descending, id ascending) and writes the first k. The row's
-// k largest are among its slices' k largest, so the result is exact and a function of the row alone.
+// top-k: a bf16 logit is a 16-bit sortable key. A row is cut into contiguous slices, one CTA each. A CTA reads its
+// slice once, 64 keys a thread into registers, and needs no histogram: K keys reach the smallest, over the warps, of a
+// warp's ceil(K / warps)-th largest THREAD maximum, so that is a lower bound T0 of the slice's K-th largest key.
+// The keys that reach T0 are few, they are ranked against each other by (key descending, id ascending), and the first
+// K are the slice's candidates, in order. Only a slice whose keys tie or crowd at T0 (more than kCand reach it) takes the
+// exact route: bisect the key range on the count of all keys, then the smallest ids among the ties. A second kernel does the
+// same over the slices' ordered candidates. The row's k largest are among its slices' k largest, so the result is
+// exact and a function of the row alone.
 //
 // draw: token = argmax over the kept candidates of logit/T + Gumbel(hash(seed, position, id)), the
 // candidates being the top_k cut to the smallest prefix whose tempered probability reaches top_p.
 // The hash (splitmix64) and the arithmetic (fp64) follow the host rule, so a row gets the same
-// token whether it is drawn alone or inside a window.
+// token whether it is drawn alone or inside a window. A warp draws a row: a lane does two candidates' exponentials
+// and logarithms, and the sums run over the candidates in order.
+//
+// Bound: the row bytes from HBM (128 rows x 248320: 63.6 MB, 9.7 us at 6.55 TB/s). The former histogram kernel
+// (keys staged in shared memory, two atomic histograms with a match per key) took 111 us there, its merge 12 us and a
+// draw of one thread a row 19.5 us.
 
 #include "common.cuh"
 
@@ -19,153 +25,163 @@ namespace tf {
 namespace {
 
 constexpr int kMaxK = 64;
-constexpr int kSliceThreads = 256, kSliceMax = 16384, kMaxSlices = 64, kMergeThreads = 1024;
+constexpr int kSliceThreads = 256, kChunks = 8;                       // a thread holds kChunks x 8 keys
+constexpr int kSliceMax = kSliceThreads * kChunks * 8 - 8;            // a slice off a 16-byte boundary takes one chunk more
+constexpr int kSliceMin = 4096;
+constexpr int kCand = 1024, kMaxSlices = 64, kMergeThreads = 128;
 
-__host__ __device__ inline int slice_len(int V) {
-    const int slices = (V + kSliceMax - 1) / kSliceMax;
-    return (((V + slices - 1) / slices) + 7) & ~7;          // a multiple of 8 entries: slices start 16-byte aligned
+// Slices are cut so that a few rows still give every SM a CTA (down to kSliceMin entries a slice, at most kMaxSlices),
+// many rows the longest slices: the result does not depend on the cut.
+__host__ __device__ inline int slice_len(int V, int rows) {
+    int slices = (V + kSliceMax - 1) / kSliceMax;
+    const int most = V / kSliceMin < kMaxSlices ? V / kSliceMin : kMaxSlices, want = (148 + rows - 1) / rows;
+    if (slices < want) slices = want < most ? want : (most > slices ? most : slices);
+    return (((V + slices - 1) / slices) + 7) & ~7;          // a multiple of 8 entries: slices of an aligned row are aligned
 }
-__host__ __device__ inline int slice_count(int V) { return (V + slice_len(V) - 1) / slice_len(V); }
+__host__ __device__ inline int slice_count(int V, int rows) { const int L = slice_len(V, rows); return (V + L - 1) / L; }
 
-__device__ __forceinline__ uint32_t sort_key(uint32_t b) { return (b & 0x8000u) ? (~b & 0xFFFFu) : (b | 0x8000u); }
 __device__ __forceinline__ uint32_t unsort_key(uint32_t k) { return (k & 0x8000u) ? (k & 0x7FFFu) : (~k & 0xFFFFu); }
+// two bf16 values -> two sortable keys: a negative value's bits are inverted, a positive one's sign bit is set
+__device__ __forceinline__ uint32_t sort_keys2(uint32_t w) {
+    const uint32_t neg = (w >> 15) & 0x00010001u;
+    return w ^ (0x80008000u | (neg * 0x7FFFu));
+}
 
-// exclusive prefix sum of one int per thread over a CTA of NT threads, fixed order
-template <int NT>
-__device__ int block_scan(int v, int* warp_tot, int& total) {
-    constexpr int NW = NT / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += n;
+// the largest T such that `count(T) >= K`, bisected over 16-bit keys (count(0) >= K must hold); `count` is block-wide
+template <class Count>
+__device__ __forceinline__ uint32_t bisect_key(int K, Count count) {
+    uint32_t T = 0;
+#pragma unroll 1
+    for (int bit = 15; bit >= 0; --bit) {
+        const uint32_t t = T | (1u << bit);
+        if (count(t) >= K) T = t;
     }
-    if (lane == 31) warp_tot[warp] = inc;
+    return T;
+}
+
+// Order of candidates: key descending, then id ascending, as one 64-bit number.
+__device__ __forceinline__ unsigned long long rank_code(uint32_t key, uint32_t id) { return ((unsigned long long)key << 32) | (0xFFFFFFFFu - id); }
+
+// The exact route, for a slice whose keys crowd: its kk largest (ties to the smallest ids) into c_s, unordered. Reads the
+// slice from memory again: a thread's registers then hold no more than the ordinary route needs.
+__device__ __noinline__ void exact_slice(const uint16_t* xr, int n, int v0, int kk, unsigned long long* c_s, int* n_s, int* scan_s) {
+    const int tid = threadIdx.x, passes = (n + kSliceThreads - 1) / kSliceThreads;
+    auto key_at = [&](int e) { return sort_keys2(xr[e]) & 0xFFFFu; };
+    const uint32_t T = bisect_key(kk, [&](uint32_t t) {
+        int mine = 0;
+        for (int e = tid; e < n; e += kSliceThreads) mine += key_at(e) >= t;
+        mine = __reduce_add_sync(0xffffffffu, mine);
+        if ((tid & 31) == 0) scan_s[tid >> 5] = mine;
+        __syncthreads();
+        int all = 0;
+        for (int w = 0; w < kSliceThreads / 32; ++w) all += scan_s[w];
+        __syncthreads();
+        return all;
+    });
+    if (tid == 0) *n_s = 0;
     __syncthreads();
-    if (warp == 0) {
-        int w = lane < NW ? warp_tot[lane] : 0, winc = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int n = __shfl_up_sync(0xffffffffu, winc, o);
-            if (lane >= o) winc += n;
+    for (int e = tid; e < n; e += kSliceThreads)
+        if (key_at(e) > T) c_s[atomicAdd(n_s, 1)] = rank_code(key_at(e), (uint32_t)(v0 + e));      // at most kk - 1
+    __syncthreads();
+    int taken = *n_s;
+    for (int i = 0; i < passes && taken < kk; ++i) {
+        const int e = i * kSliceThreads + tid;
+        const bool tie = e < n && key_at(e) == T;
+        const unsigned m = __ballot_sync(0xffffffffu, tie);
+        if ((tid & 31) == 0) scan_s[tid >> 5] = __popc(m);
+        __syncthreads();
+        int at = taken + __popc(m & ((1u << (tid & 31)) - 1u));
+        for (int w = 0; w < kSliceThreads / 32; ++w) {
+            if (w < (tid >> 5)) at += scan_s[w];
+            taken += scan_s[w];
         }
-        if (lane < NW) warp_tot[lane] = winc - w;
-        if (lane == 31) warp_tot[32] = winc;
+        if (tie && at < kk) c_s[at] = rank_code(T, (uint32_t)(v0 + e));
+        __syncthreads();
     }
-    __syncthreads();
-    const int base = warp_tot[warp];
-    total = warp_tot[32];
-    __syncthreads();
-    return base + inc - v;
 }
 
-// One histogram pass over the staged keys: bin = byte `shift` of the keys that pass `keep`; lanes of a
-// warp that hit the same bin add once (logits crowd into a few exponents). Then the bin holding the
-// K-th largest is found: found[0] = bin, found[1] = entries in higher bins.
-template <class Keep>
-__device__ void select_byte(const uint16_t* keys, int n, int shift, int K, int above0, unsigned* hist, int* warp_tot, int* found,
-                            Keep keep) {
-    const int tid = threadIdx.x;
-    hist[tid] = 0;
-    __syncthreads();
-    const int padded = (n + kSliceThreads - 1) / kSliceThreads * kSliceThreads;
-    for (int i = tid; i < padded; i += kSliceThreads) {
-        const uint32_t key = i < n ? keys[i] : 0u;
-        const int bin = (i < n && keep(key)) ? (int)((key >> shift) & 0xFFu) : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, bin);
-        if (bin >= 0 && (tid & 31) == __ffs(peers) - 1) atomicAdd(&hist[bin], (unsigned)__popc(peers));
-    }
-    __syncthreads();
-    // entries in bins above mine: an exclusive prefix sum over the bins in descending order
-    const int mine = (int)hist[255 - tid];
-    int total;
-    const int above = above0 + block_scan<kSliceThreads>(mine, warp_tot, total);
-    if (above < K && above + mine >= K) { found[0] = 255 - tid; found[1] = above; }
-    __syncthreads();
-}
-
-__global__ void __launch_bounds__(kSliceThreads) topk_slice_kernel(const __nv_bfloat16* x, size_t row_stride, int V, int K, uint2* cand) {
-    __shared__ __align__(16) uint16_t keys[kSliceMax];
-    __shared__ unsigned hist[256];
-    __shared__ int found[2];
-    __shared__ int warp_tot[33];
+__global__ void __launch_bounds__(kSliceThreads, 4) topk_slice_kernel(const __nv_bfloat16* x, size_t row_stride, int V, int K, int L,
+                                                                   unsigned long long* cand) {
+    __shared__ unsigned long long c_s[kCand];
+    __shared__ int n_s, scan_s[kSliceThreads / 32 + 1];
     pdl_launch_dependents();
     pdl_wait();
-    const int tid = threadIdx.x, row = blockIdx.y, L = slice_len(V);
+    const int tid = threadIdx.x, row = blockIdx.y;
     const int v0 = blockIdx.x * L, n = min(L, V - v0);
     const uint16_t* xr = reinterpret_cast<const uint16_t*>(x) + (size_t)row * row_stride + v0;
-    uint2* out = cand + ((size_t)row * gridDim.x + blockIdx.x) * K;
+    unsigned long long* out = cand + ((size_t)row * gridDim.x + blockIdx.x) * K;
     const int kk = min(K, n);                                   // a short slice yields all it has
-    for (int j = tid + kk; j < K; j += kSliceThreads) out[j] = make_uint2(0u, 0x7FFFFFFFu);   // ranks behind every real entry
-
-    if ((reinterpret_cast<uintptr_t>(xr) & 15) == 0) {
-        for (int i = tid * 8; i < n; i += kSliceThreads * 8) {
-            const uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    // chunks of 16 aligned bytes that hold the slice: chunk c has entries 8c - off .. 8c - off + 7
+    const int off = (int)((reinterpret_cast<uintptr_t>(xr) & 15) >> 1), chunks = (n + off + 7) >> 3;
+    uint4 key[kChunks];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (i + 2 * j < n) keys[i + 2 * j] = (uint16_t)sort_key(w[j] & 0xFFFFu);
-                if (i + 2 * j + 1 < n) keys[i + 2 * j + 1] = (uint16_t)sort_key(w[j] >> 16);
+    for (int i = 0; i < kChunks; ++i) {
+        const int c = i * kSliceThreads + tid, e0 = 8 * c - off;
+        if (c < chunks && e0 >= 0 && e0 + 8 <= n) key[i] = __ldcs(reinterpret_cast<const uint4*>(xr + e0));
+    }
+    if (tid == 0) n_s = 0;
+    uint32_t top2 = 0;
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+        const int c = i * kSliceThreads + tid, e0 = 8 * c - off;
+        if (c < chunks && e0 >= 0 && e0 + 8 <= n) {
+            key[i] = make_uint4(sort_keys2(key[i].x), sort_keys2(key[i].y), sort_keys2(key[i].z), sort_keys2(key[i].w));
+        } else {                                                // an end chunk, or none: entries outside the slice are key 0
+            uint32_t w[4] = {0u, 0u, 0u, 0u};
+            if (c < chunks)
+                for (int j = 0; j < 8; ++j)
+                    if (e0 + j >= 0 && e0 + j < n) w[j >> 1] |= (sort_keys2(xr[e0 + j]) & 0xFFFFu) << (16 * (j & 1));
+            key[i] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        top2 = __vmaxu2(top2, __vmaxu2(__vmaxu2(key[i].x, key[i].y), __vmaxu2(key[i].z, key[i].w)));
+    }
+    const uint32_t top = max(top2 & 0xFFFFu, top2 >> 16);
+    // T0: each warp's ceil(kk / warps)-th largest thread maximum, the smallest of them over the warps: kk keys reach it.
+    // (Fewer threads than that hold entries only in a slice of less than 8 * (kk + warps): T0 is then 0, every entry a candidate.)
+    constexpr int kWarps = kSliceThreads / 32;
+    {
+        uint32_t left = top + 1, reached = 0;                   // 0: taken
+        for (int r = 0; r < kk; r += kWarps) {
+            reached = __reduce_max_sync(0xffffffffu, left);
+            if ((tid & 31) == __ffs(__ballot_sync(0xffffffffu, left == reached)) - 1) left = 0;
+        }
+        if ((tid & 31) == 0) scan_s[tid >> 5] = (int)(reached == 0 ? 0u : reached - 1);
+    }
+    __syncthreads();
+    uint32_t T = 0xFFFFu;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) T = min(T, (uint32_t)scan_s[w]);
+    if (top >= T) {
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+            const uint32_t m = __vmaxu2(__vmaxu2(key[i].x, key[i].y), __vmaxu2(key[i].z, key[i].w));
+            if (max(m & 0xFFFFu, m >> 16) < T) continue;
+            const uint32_t w[4] = {key[i].x, key[i].y, key[i].z, key[i].w};
+            const int e0 = 8 * (i * kSliceThreads + tid) - off;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t k = (w[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
+                if (k >= T && (unsigned)(e0 + j) < (unsigned)n) {
+                    const int at = atomicAdd(&n_s, 1);
+                    if (at < kCand) c_s[at] = rank_code(k, (uint32_t)(v0 + e0 + j));
+                }
             }
         }
-    } else {
-        for (int i = tid; i < n; i += kSliceThreads) keys[i] = (uint16_t)sort_key(xr[i]);
     }
     __syncthreads();
-
-    select_byte(keys, n, 8, kk, 0, hist, warp_tot, found, [](uint32_t) { return true; });
-    const uint32_t hb = (uint32_t)found[0];
-    const int above_hb = found[1];
-    __syncthreads();
-    select_byte(keys, n, 0, kk, above_hb, hist, warp_tot, found, [hb](uint32_t key) { return (key >> 8) == hb; });
-    const uint32_t T = (hb << 8) | (uint32_t)found[0];
-    const int above = found[1], need = kk - above;              // entries strictly above T; ties still wanted
-
-    // everything above T, then the first `need` ties, both in id order
-    const int per = (n + kSliceThreads - 1) / kSliceThreads;
-    const int lo = min(n, tid * per), hi = min(n, lo + per);
-    int n_above = 0, n_tie = 0;
-    for (int i = lo; i < hi; ++i) {
-        const uint32_t key = keys[i];
-        n_above += key > T;
-        n_tie += key == T;
+    int have = n_s;
+    if (have > kCand) {
+        __syncthreads();
+        exact_slice(xr, n, v0, kk, c_s, &n_s, scan_s);
+        have = kk;
     }
-    int total;
-    int at_above = block_scan<kSliceThreads>(n_above, warp_tot, total);
-    int at_tie = block_scan<kSliceThreads>(n_tie, warp_tot, total);
-    for (int i = lo; i < hi; ++i) {
-        const uint32_t key = keys[i];
-        if (key > T) {
-            out[at_above++] = make_uint2(key, (uint32_t)(v0 + i));
-        } else if (key == T) {
-            if (at_tie < need) out[above + at_tie] = make_uint2(key, (uint32_t)(v0 + i));
-            ++at_tie;
-        }
-    }
-}
-
-// One CTA per row: rank the slices' candidates by (key descending, id ascending); ranks are distinct.
-__global__ void __launch_bounds__(kMergeThreads) topk_merge_kernel(const uint2* cand, int n, int K, int* idx_out, float* val_out) {
-    __shared__ uint2 c[kMaxSlices * kMaxK];
-    pdl_launch_dependents();
-    pdl_wait();
-    const int row = blockIdx.x;
-    for (int i = threadIdx.x; i < n; i += kMergeThreads) c[i] = cand[(size_t)row * n + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kMergeThreads) {
-        const uint2 me = c[i];
-        if (me.y == 0x7FFFFFFFu) continue;
+    for (int i = tid; i < have; i += kSliceThreads) {
+        const unsigned long long me = c_s[i];
         int rank = 0;
-        for (int j = 0; j < n; ++j) {
-            const uint2 o = c[j];
-            rank += (o.x > me.x) || (o.x == me.x && o.y < me.y);
-        }
-        if (rank < K) {
-            idx_out[(size_t)row * K + rank] = (int)me.y;
-            val_out[(size_t)row * K + rank] = __uint_as_float(unsort_key(me.x) << 16);
-        }
+        for (int j = 0; j < have; ++j) rank += c_s[j] > me;
+        if (rank < kk) out[rank] = me;
     }
+    for (int j = tid + kk; j < K; j += kSliceThreads) out[j] = 0ull;       // ranks behind every real entry
 }
 
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
@@ -174,41 +190,134 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
     return x ^ (x >> 31);
 }
 
-// One thread per row: candidates are few (<= 64) and the rule is a chain of fp64 operations.
-__global__ void sample_kernel(const int* idx, const float* val, int width, const long long* positions,
-                              unsigned long long seed, double temperature, int top_k, double top_p, int* tokens, int rows) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row >= rows) return;
-    const int* ids = idx + (size_t)row * width;
-    const float* vals = val + (size_t)row * width;        // already ordered (value desc, id asc)
-    const int k = max(1, min(top_k > 0 ? top_k : width, width));
-    const double t = fmax(temperature, 1e-6);
-    const double top = (double)vals[0] / t;
+struct Draw {
+    const long long* positions;
+    unsigned long long seed;
+    double temperature, top_p;
+    int top_k;
+    int* tokens;
+};
+
+// One warp draws a row from its candidates, ordered by (value desc, id asc). Lane l holds candidates l and l + 32; the
+// sums add the candidates one by one in order (the host rule's order), fetched from their lanes.
+__device__ __forceinline__ int draw_row(const int (&id)[2], const float (&val)[2], int width, long long position, const Draw& d) {
+    const int lane = threadIdx.x & 31;
+    const int k = max(1, min(d.top_k > 0 ? d.top_k : width, width));
+    const double t = fmax(d.temperature, 1e-6);
+    const double s0 = (double)val[0] / t, s1 = (double)val[1] / t;
+    const double top = __shfl_sync(0xffffffffu, s0, 0);
     int keep = k;
-    if (top_p > 0.0 && top_p < 1.0) {
+    if (d.top_p > 0.0 && d.top_p < 1.0) {
+        const double e0 = lane < k ? exp(s0 - top) : 0.0, e1 = lane + 32 < k ? exp(s1 - top) : 0.0;
         double denom = 0.0;
-        for (int j = 0; j < k; ++j) denom += exp((double)vals[j] / t - top);
+        for (int j = 0; j < k; ++j) denom += __shfl_sync(0xffffffffu, j < 32 ? e0 : e1, j & 31);
+        const double p0 = e0 / denom, p1 = e1 / denom;
         double cum = 0.0;
         int below = 0;
         for (int j = 0; j < k; ++j) {
-            cum += exp((double)vals[j] / t - top) / denom;
-            below += cum < top_p;
+            cum += __shfl_sync(0xffffffffu, j < 32 ? p0 : p1, j & 31);
+            below += cum < d.top_p;
         }
         keep = min(k, below + 1);
     }
-    const unsigned long long h0 = mix64(seed + 0x9E3779B97F4A7C15ull);
-    const unsigned long long h1 = mix64(h0 ^ ((unsigned long long)positions[row] * 0xD1B54A32D192ED03ull));
+    const unsigned long long h0 = mix64(d.seed + 0x9E3779B97F4A7C15ull);
+    const unsigned long long h1 = mix64(h0 ^ ((unsigned long long)position * 0xD1B54A32D192ED03ull));
     double best = -INFINITY;
-    int pick = ids[0];
-    for (int j = 0; j < keep; ++j) {
-        const unsigned long long h = mix64(h1 ^ (unsigned long long)(long long)ids[j]);
-        const double u = (double)(h >> 11) * 0x1.0p-53 + 0x1.0p-54;
-        const double score = (double)vals[j] / t - log(-log(u));
-        if (score > best) { best = score; pick = ids[j]; }
+    int at = 0x7FFFFFFF, pick = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (lane + 32 * h < keep) {
+            const unsigned long long hash = mix64(h1 ^ (unsigned long long)(long long)id[h]);
+            const double u = (double)(hash >> 11) * 0x1.0p-53 + 0x1.0p-54;
+            const double score = (h ? s1 : s0) - log(-log(u));
+            if (score > best) { best = score; at = lane + 32 * h; pick = id[h]; }
+        }
     }
-    tokens[row] = pick;
+    // the first candidate of the largest score, as a scan in order would keep it
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, at, o), op = __shfl_xor_sync(0xffffffffu, pick, o);
+        if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; pick = op; }
+    }
+    const int first = __shfl_sync(0xffffffffu, id[0], 0);
+    return at == 0x7FFFFFFF ? first : pick;                    // no score above -inf: the first candidate
+}
+
+// One CTA per row: the slices' candidates that reach a lower bound of the K-th largest, ranked; with `d.tokens` the row's
+// token is drawn from them in the same launch (idx_out and val_out may then be null).
+__global__ void __launch_bounds__(kMergeThreads) topk_merge_kernel(const unsigned long long* cand, int n, int K, int* idx_out, float* val_out,
+                                                                   const Draw d) {
+    __shared__ unsigned long long c_s[kMaxSlices * kMaxK];
+    __shared__ unsigned long long best_s[kMaxK];
+    __shared__ int n_s;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, slices = n / K;
+    const unsigned long long* c = cand + (size_t)row * n;
+    if (tid == 0) n_s = 0;
+    // every slice's list is in order: with the first ceil(K / slices) of each, K candidates reach the smallest of those
+    // lists' last entries (0, below every real entry, where a slice has fewer)
+    const int at = (K + slices - 1) / slices - 1;
+    unsigned long long T = ~0ull;
+    for (int s = lane; s < slices; s += 32) T = min(T, c[s * K + at]);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) T = min(T, __shfl_xor_sync(0xffffffffu, T, o));
+    __syncthreads();
+    constexpr int U = 4;                                       // loads in flight
+    for (int i0 = tid; i0 < n; i0 += U * kMergeThreads) {
+        unsigned long long mine[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) mine[u] = i0 + u * kMergeThreads < n ? c[i0 + u * kMergeThreads] : 0ull;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (mine[u] != 0ull && mine[u] >= T) c_s[atomicAdd(&n_s, 1)] = mine[u];
+    }
+    __syncthreads();
+    const int have = n_s;
+    for (int i = tid; i < have; i += kMergeThreads) {
+        const unsigned long long me = c_s[i];
+        int rank = 0;
+        for (int j = 0; j < have; ++j) rank += c_s[j] > me;
+        if (rank < K) {
+            best_s[rank] = me;
+            if (idx_out != nullptr) {
+                idx_out[(size_t)row * K + rank] = (int)(0xFFFFFFFFu - (uint32_t)me);
+                val_out[(size_t)row * K + rank] = __uint_as_float(unsort_key((uint32_t)(me >> 32)) << 16);
+            }
+        }
+    }
+    if (d.tokens == nullptr) return;
+    __syncthreads();
+    if (tid >= 32) return;
+    int id[2];
+    float val[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const unsigned long long c = tid + 32 * h < K ? best_s[tid + 32 * h] : best_s[0];
+        id[h] = (int)(0xFFFFFFFFu - (uint32_t)c);
+        val[h] = __uint_as_float(unsort_key((uint32_t)(c >> 32)) << 16);
+    }
+    const int token = draw_row(id, val, K, d.positions[row], d);
+    if (tid == 0) d.tokens[row] = token;
+}
+
+// The draw alone, from candidates already ordered: a warp per row.
+__global__ void sample_kernel(const int* idx, const float* val, int width, const Draw d, int rows) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    int id[2];
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int j = lane + 32 * h < width ? lane + 32 * h : 0;
+        id[h] = idx[(size_t)row * width + j];
+        v[h] = val[(size_t)row * width + j];
+    }
+    const int token = draw_row(id, v, width, d.positions[row], d);
+    if (lane == 0) d.tokens[row] = token;
 }
 
 }  // namespace
@@ -218,25 +327,26 @@ extern "C" {
 
 size_t tf_topk_scratch_bytes(int rows, int vocab, int k) {
     if (rows < 1 || vocab < 1 || k < 1 || k > tf::kMaxK) return 0;
-    return (size_t)rows * tf::slice_count(vocab) * k * sizeof(uint2);
+    return (size_t)rows * tf::slice_count(vocab, rows) * k * sizeof(unsigned long long);
 }
 
-int tf_topk_rows(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, void* scratch,
-                 size_t scratch_bytes, void* stream) {
+static int topk(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, tf::Draw draw, void* scratch,
+                size_t scratch_bytes, void* stream) {
     if (rows < 1 || rows > 65535 || vocab < 1 || k < 1 || k > tf::kMaxK || k > vocab || row_stride < (size_t)vocab) return TF_EINVAL;
-    if (!x || !idx || !val) return TF_EINVAL;
-    const int slices = tf::slice_count(vocab);
+    if (!x || (!idx != !val) || (!idx && !draw.tokens)) return TF_EINVAL;
+    if (reinterpret_cast<uintptr_t>(x) & 1) return TF_EALIGN;
+    const int slices = tf::slice_count(vocab, rows);
     if (slices > tf::kMaxSlices) return TF_EINVAL;
     if (!scratch || scratch_bytes < tf_topk_scratch_bytes(rows, vocab, k)) return TF_ESCRATCH;
     if (reinterpret_cast<uintptr_t>(scratch) & 7) return TF_EALIGN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    void* a1[] = {&x, &row_stride, &vocab, &k, &scratch};
+    int len = tf::slice_len(vocab, rows), n = slices * k;
+    void* a1[] = {&x, &row_stride, &vocab, &k, &len, &scratch};
     if (tf::launch_pdl((const void*)tf::topk_slice_kernel, dim3(slices, rows), dim3(tf::kSliceThreads), 0, st, a1) != cudaSuccess) {
         cudaGetLastError();
         return TF_ECUDA;
     }
-    int n = slices * k;
-    void* a2[] = {&scratch, &n, &k, &idx, &val};
+    void* a2[] = {&scratch, &n, &k, &idx, &val, &draw};
     if (tf::launch_pdl((const void*)tf::topk_merge_kernel, dim3(rows), dim3(tf::kMergeThreads), 0, st, a2) != cudaSuccess) {
         cudaGetLastError();
         return TF_ECUDA;
@@ -244,11 +354,25 @@ int tf_topk_rows(const void* x, size_t row_stride, int rows, int vocab, int k, i
     return TF_OK;
 }
 
+int tf_topk_rows(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, void* scratch,
+                 size_t scratch_bytes, void* stream) {
+    if (!idx) return TF_EINVAL;
+    return topk(x, row_stride, rows, vocab, k, idx, val, tf::Draw{}, scratch, scratch_bytes, stream);
+}
+
+int tf_topk_sample_rows(const void* x, size_t row_stride, int rows, int vocab, int k, const long long* positions, unsigned long long seed,
+                        double temperature, int top_k, double top_p, int* tokens, void* scratch, size_t scratch_bytes, void* stream) {
+    if (!positions || !tokens) return TF_EINVAL;
+    return topk(x, row_stride, rows, vocab, k, nullptr, nullptr, tf::Draw{positions, seed, temperature, top_p, top_k, tokens}, scratch,
+                scratch_bytes, stream);
+}
+
 int tf_sample_rows(const int* idx, const float* val, int width, const long long* positions, unsigned long long seed,
                    double temperature, int top_k, double top_p, int* tokens, int rows, void* stream) {
     if (rows < 1 || width < 1 || width > tf::kMaxK || !idx || !val || !positions || !tokens) return TF_EINVAL;
-    void* args[] = {&idx, &val, &width, &positions, &seed, &temperature, &top_k, &top_p, &tokens, &rows};
-    if (tf::launch_pdl((const void*)tf::sample_kernel, dim3((rows + 63) / 64), dim3(64), 0, static_cast<cudaStream_t>(stream), args) !=
+    tf::Draw draw{positions, seed, temperature, top_p, top_k, tokens};
+    void* args[] = {&idx, &val, &width, &draw, &rows};
+    if (tf::launch_pdl((const void*)tf::sample_kernel, dim3((rows + 3) / 4), dim3(128), 0, static_cast<cudaStream_t>(stream), args) !=
         cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
 }

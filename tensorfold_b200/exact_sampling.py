@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .topk import MAX_K, topk_rows
+from .topk import MAX_K, rows_of, topk_rows
 
 MARGIN = 8     # candidates beyond top_k read from the top-k kernel, so tied values resolve by id
 
@@ -54,12 +54,17 @@ def choose_rows(values, ids, positions: Sequence[int], s: Sampling) -> list[int]
     return [int(t) for t in tokens.cpu()]
 
 
+def candidates(vocab: int, s: Sampling) -> int:
+    """Entries of a row the draw looks at."""
+
+    return min(vocab, (int(s.top_k) if s.top_k else MAX_K - MARGIN) + MARGIN, MAX_K)
+
+
 def top_candidates(logits: torch.Tensor, s: Sampling) -> tuple[torch.Tensor, torch.Tensor]:
     """The rows' top ``top_k + MARGIN`` (ids, values), ordered by (value desc, id asc)."""
 
     vocab = logits.shape[-1]
-    count = min(vocab, (int(s.top_k) if s.top_k else MAX_K - MARGIN) + MARGIN, MAX_K)
-    return topk_rows(logits.reshape(-1, vocab), count)
+    return topk_rows(logits.reshape(-1, vocab), candidates(vocab, s))
 
 
 def sample_rows(logits: torch.Tensor, positions, s: Sampling | None, *, top: tuple | None = None) -> torch.Tensor:
@@ -74,17 +79,24 @@ def sample_rows(logits: torch.Tensor, positions, s: Sampling | None, *, top: tup
         return topk_rows(logits, 1)[0].reshape(rows)
     if not 0 < int(s.top_k) <= MAX_K - MARGIN:
         raise ValueError(f"sample_rows: top_k must be in 1..{MAX_K - MARGIN} (the radix top-k holds {MAX_K} candidates)")
-    idx, val = top if top is not None else top_candidates(logits, s)
     if not torch.is_tensor(positions):
         positions = torch.tensor(list(positions), dtype=torch.int64)
     positions = positions.to(device=logits.device, dtype=torch.int64)
     if positions.shape != (rows,):
         raise ValueError("sample_rows: one position per row")
     tokens = torch.empty(rows, dtype=torch.int32, device=logits.device)
+    rule = (int(s.seed) & 0xFFFFFFFFFFFFFFFF, float(s.temperature), int(s.top_k), float(s.top_p), tokens)
+    lib = _lib.load()
     with _lib.on(logits.device):
-        _lib.check(_lib.load().tf_sample_rows(idx, val, idx.shape[1], positions,
-                                              int(s.seed) & 0xFFFFFFFFFFFFFFFF, float(s.temperature), int(s.top_k),
-                                              float(s.top_p), tokens, rows, _lib.stream()), "sample_rows")
+        if top is not None:
+            idx, val = top
+            _lib.check(lib.tf_sample_rows(idx, val, idx.shape[1], positions, *rule, rows, _lib.stream()), "sample_rows")
+        else:
+            x, count = rows_of(logits), candidates(logits.shape[-1], s)
+            need = lib.tf_topk_scratch_bytes(rows, x.shape[1], count)
+            scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+            _lib.check(lib.tf_topk_sample_rows(x, x.stride(0), rows, x.shape[1], count, positions, *rule, scratch, need, _lib.stream()),
+                       "sample_rows")
     return tokens
 
 

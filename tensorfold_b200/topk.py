@@ -14,15 +14,20 @@ from . import _lib
 MAX_K = 64
 
 
+def rows_of(x: torch.Tensor) -> torch.Tensor:
+    """``x`` as 2-D bf16 rows with unit inner stride, the form the kernels read."""
+
+    if x.dtype != torch.bfloat16:
+        x = x.to(torch.bfloat16)
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+    return x2 if x2.stride(1) == 1 else x2.contiguous()
+
+
 def topk_rows(x: torch.Tensor, k: int, scratch: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
     """(indices [R, k] int32, values [R, k] float32) of each row's k largest, value desc then id asc."""
 
     _lib.need_cuda(x)
-    if x.dtype != torch.bfloat16:
-        x = x.to(torch.bfloat16)
-    x2 = x.reshape(-1, x.shape[-1])
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
+    x2 = rows_of(x)
     rows, vocab = x2.shape
     k = int(k)
     if not 1 <= k <= MAX_K or k > vocab:
