@@ -59,21 +59,26 @@ __host__ __device__ constexpr int nibble_quad(int j) { return ((j >> 1) & 1) * 2
 __host__ __device__ constexpr int tile_k(int t, int s, int quad) { return 32 * (s >> 1) + 8 * t + 4 * (s & 1) + quad; }
 
 // One instantiation per row bucket: MB blocks of 8 rows, KTS k tiles a pipeline stage, T column tiles per
-// consumer warp (they share the activation loads), CTAS CTAs of the kernel that fit one SM.
-template <int G_, int MB_, int KTS_, int T_, int CTAS_>
+// consumer warp (they share the activation loads), HALVES passes over the weights, each for its own MB * 8 rows of a
+// bucket of HALVES times as many.
+template <int G_, int MB_, int KTS_, int T_, int HALVES_ = 1>
 struct Cfg {
-    static constexpr int G = G_, MB = MB_, KTS = KTS_, T = T_, CTAS = CTAS_;
+    static constexpr int G = G_, MB = MB_, KTS = KTS_, T = T_, HALVES = HALVES_;
     static constexpr int REC = rec_bytes(G);
     static constexpr int GPT = 64 / G;                 // groups per k tile
-    static constexpr int ROWS = MB * 8;                // = tf_padded_rows(M) for every M of the bucket
-    static constexpr int XTILE = ROWS * (128 + 4 * GPT);   // packed activation bytes per k tile
+    static constexpr int ROWS = MB * 8;                // rows of a pass; ROWS * HALVES = tf_padded_rows(M) for every M of the bucket
+    static constexpr int XTILE = ROWS * (128 + 4 * GPT);   // packed activation bytes per k tile and pass
     static constexpr int W_BYTES = kWarps * KTS * REC;
     static constexpr int X_BYTES = KTS * XTILE;
     static constexpr int STAGE_BYTES = ((W_BYTES + X_BYTES + 127) / 128) * 128;
     static constexpr int CW = kWarps / T;               // consumer warps
-    static constexpr int THREADS = (CW + 1) * 32;       // consumers + producer warp
-    // the ring takes the SM's shared memory (1 KB a CTA belongs to the system), split between CTAS CTAs
-    static constexpr int BUDGET = (CTAS == 2 ? 113 : 226) * 1024 - 512;
+    // With 64 rows the eight consumer warps want more than the 168 registers a thread that nine warps get (the allocation
+    // is by four warps): the producer's warp group hands its own over (256 x 216 + 128 x 72 = the 384 x 168 of the launch).
+    static constexpr bool REGS = MB >= 8;
+    static constexpr int THREADS = REGS ? 384 : (CW + 1) * 32;       // consumers + producer warp
+    static_assert(!REGS || CW == 8, "two consumer warp groups");
+    // the ring takes the SM's shared memory (1 KB belongs to the system)
+    static constexpr int BUDGET = 226 * 1024 - 512;
     static constexpr int STAGES = BUDGET / (STAGE_BYTES + 16) > 12 ? 12 : BUDGET / (STAGE_BYTES + 16);
     static constexpr int SMEM = STAGES * STAGE_BYTES + 2 * STAGES * 8 + 128;
     static_assert(STAGES >= 2, "the ring needs at least two stages");
@@ -100,7 +105,9 @@ struct Args {
     const uint8_t* w;
     void* y;
     uint32_t* epochs;
+    uint32_t* flags;
     float* slots;
+    float* packets;
     int* status;
     int M, N, K;
     int f32_out;
@@ -137,15 +144,28 @@ struct Args {
 __host__ __device__ inline int range_begin(int cta, int total) { return (int)((unsigned)cta * (unsigned)total / (unsigned)kWorkers); }
 
 constexpr size_t kSlotFloats = (size_t)TF_QMM_MAX_ROWS * kCols;
-// scratch: [ticket words of the prefill kernel][parked segments, one slot of 2 x 128 x 256 floats a worker]
-//          [launch numbers, one a worker]
+// scratch: [ticket words of the wide-row kernel][parked segments, two slots of 128 x 256 floats a worker]
+//          [launch numbers, one a worker][ready flags][packets]
 constexpr size_t kEpochOffset = TF_QMM_COUNTER_BYTES + 2 * kWorkers * kSlotFloats * sizeof(float);
-constexpr size_t kScratchBytes = kEpochOffset + 1024;
+// ready flags of the parked segments (two a worker), behind the launch numbers; each in a 128-byte line of its own worker
+constexpr size_t kFlagOffset = kEpochOffset + 1024;
+constexpr size_t kFlagStride = 32;      // words
+// the self-tagged packets of launches of up to 8 rows have a place that nothing else writes: a stale word there is an older tag
+constexpr size_t kPacketOffset = kFlagOffset + kWorkers * kFlagStride * sizeof(uint32_t);
+constexpr size_t kPacketFloats = (size_t)2 * 8 * kCols;               // a worker's segment of 8 rows, half values, half tags
+constexpr size_t kScratchBytes = kPacketOffset + kWorkers * kPacketFloats * sizeof(float);
 
 // 16-byte load that is performed every time it is executed (a polled location)
 __device__ __forceinline__ float4 ld_volatile16(const float4* p) {
     float4 v;
     asm volatile("ld.volatile.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) { asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -161,8 +181,14 @@ __device__ __forceinline__ float4 ld_volatile16(const float4* p) {
 // adds them in worker order, which is k order, and writes the output. No tickets, flags or fences, one
 // round trip on the critical path, and nothing to reset. The launch number is the worker's own counter in scratch, advanced once
 // per launch before dependents may start, so every worker of a launch holds the same number.
+//
+// Above 8 rows a segment is 16 to 128 KB, and one worker that fetches up to nine of them in turn was half of the
+// launch (5120 x 4096 at 128 rows: 74 us). There every worker of a cut block parks its segment (plain values, then a
+// fence and a ready flag that carries the launch number), and the block's workers share the sum: each adds all the
+// segments of every nseg-th accumulator unit, in k order from the first segment on, and writes those outputs. All parking comes
+// before any waiting, and a launch's workers are all resident, so the waits end.
 template <class C, bool MULTI>
-__global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) {
+__global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
     constexpr int MB = C::MB, KTS = C::KTS, STAGES = C::STAGES, CW = C::CW, T = C::T, NC = CW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ uint32_t epoch_s;
@@ -201,48 +227,36 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
     __syncthreads();
     pdl_launch_dependents();     // the next kernel may be scheduled; it still waits for this one's memory
 
-    if (warp == CW) {
+    if (warp >= CW) {
+        if constexpr (C::REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         // ------------------------------- producer: one thread ----------------------------------
         // Weights never change during a forward, so the first ring of weight copies is issued before
         // waiting for the previous kernel; the activations (its output) follow after the wait.
-        if (lane == 0 && begin < end) {
-            int s = 0, issued = 0;
-            uint32_t phase = 1;
+        if (warp == CW && lane == 0 && begin < end) {
             auto picked = [&](int q) { return (MULTI && a.prob_sel) ? a.prob_sel[q] : q; };
-            int early_kt0[STAGES], early_nkt[STAGES];
-            bool waited = multi;
-            int it = begin;
-            while (it < end) {
-                const int gb = it / SPB, pq = MULTI ? gb / CB : 0, cb = gb - pq * CB;
-                const int cb_begin = gb * SPB, seg_end = min(cb_begin + SPB, end);
-                const uint8_t* wbase = a.w + (multi ? (size_t)a.prob_expert[picked(pq)] * a.w_stride : 0) +
-                                       (size_t)cb * KT * (kWarps * C::REC);
-                const uint8_t* xbase = a.xp + (multi ? (size_t)picked(pq) * a.xp_stride : 0);
-                const int kt_end = min(KT, (seg_end - cb_begin) * item_tiles);
-                for (int kt0 = (it - cb_begin) * item_tiles; kt0 < kt_end; kt0 += KTS) {
-                    const int nkt = min(KTS, kt_end - kt0);
-                    if (issued == STAGES && !waited) {
-                        pdl_wait();
-                        for (int e = 0; e < STAGES; ++e)
-                            bulk_g2s(smem_u32(stage0 + e * C::STAGE_BYTES + C::W_BYTES),
-                                     a.xp + (size_t)early_kt0[e] * C::XTILE, (uint32_t)(early_nkt[e] * C::XTILE), full_bar(e));
-                        waited = true;
-                    }
-                    mbar_wait(empty_bar(s), phase, a.status);
-                    uint8_t* sb = stage0 + s * C::STAGE_BYTES;
-                    const uint32_t wbytes = (uint32_t)(nkt * kWarps * C::REC), xbytes = (uint32_t)(nkt * C::XTILE);
-                    mbar_arrive_expect_tx(full_bar(s), wbytes + xbytes);
-                    bulk_g2s(smem_u32(sb), wbase + (size_t)kt0 * (kWarps * C::REC), wbytes, full_bar(s));
-                    if (issued == 0) stamp(tr, 1);
-                    if (waited) bulk_g2s(smem_u32(sb + C::W_BYTES), xbase + (size_t)kt0 * C::XTILE, xbytes, full_bar(s));
-                    else { early_kt0[issued] = kt0; early_nkt[issued] = nkt; }
-                    ++issued;
-                    if (++s == STAGES) { s = 0; phase ^= 1; }
+            // walks the range's pipeline stages: passes over the rows, items, k tiles of an item's segment
+            struct Walk {
+                int half, it, kt0, kt_end, gb, begin, end, SPB, KT, item_tiles;
+                __device__ void open() {                             // the segment that starts at item `it`
+                    gb = it / SPB;
+                    const int cb_begin = gb * SPB, seg_end = min(cb_begin + SPB, end);
+                    kt0 = (it - cb_begin) * item_tiles;
+                    kt_end = min(KT, (seg_end - cb_begin) * item_tiles);
                 }
-                it = seg_end;
-            }
-            stamp(tr, 7);
-            if (a.next_w != nullptr) {
+                __device__ bool valid() const { return half < C::HALVES; }
+                __device__ int nkt() const { return min(KTS, kt_end - kt0); }
+                __device__ void next() {
+                    kt0 += KTS;
+                    if (kt0 < kt_end) return;
+                    it = min((gb + 1) * SPB, end);
+                    if (it == end) { ++half; it = begin; }
+                    open();
+                }
+            };
+            bool prefetched = MULTI;
+            auto prefetch_next = [&] {
+                prefetched = true;
+                if (a.next_w == nullptr) return;
                 // where this worker's range of the next matmul starts (its items are cut like this one's)
                 const int nKT = a.next_K >> 6, nCB = (a.next_N + kCols - 1) / kCols, nIT = item_tiles_for(nCB, nKT), nSPB = (nKT + nIT - 1) / nIT;
                 const int ntotal = nCB * nSPB;
@@ -257,16 +271,60 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
                     const uint32_t piece = (uint32_t)(len - off < 32768 ? len - off : 32768);
                     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.next_w + at + off), "r"(piece) : "memory");
                 }
-            }
-            if (!waited) {
+            };
+            Walk w{0, begin, 0, 0, 0, begin, end, SPB, KT, item_tiles};
+            w.open();
+            Walk x = w;
+            int ws = 0, xs = 0, ahead = 0;                            // stages whose weights are under way and activations are not
+            uint32_t phase = 1;
+            auto issue_w = [&] {
+                const int pq = MULTI ? w.gb / CB : 0, cb = w.gb - pq * CB, nkt = w.nkt();
+                const uint8_t* wbase = a.w + (multi ? (size_t)a.prob_expert[picked(pq)] * a.w_stride : 0) + (size_t)cb * KT * (kWarps * C::REC);
+                mbar_wait(empty_bar(ws), phase, a.status);
+                const uint32_t wbytes = (uint32_t)(nkt * kWarps * C::REC);
+                mbar_arrive_expect_tx(full_bar(ws), wbytes + (uint32_t)(nkt * C::XTILE));
+                bulk_g2s(smem_u32(stage0 + ws * C::STAGE_BYTES), wbase + (size_t)w.kt0 * (kWarps * C::REC), wbytes, full_bar(ws));
+                if (++ws == STAGES) { ws = 0; phase ^= 1; }
+                w.next();
+                ++ahead;
+            };
+            auto issue_x = [&] {
+                const uint8_t* xbase = a.xp + (multi ? (size_t)picked(x.gb / CB) * a.xp_stride : 0);
+                const uint32_t dst = smem_u32(stage0 + xs * C::STAGE_BYTES + C::W_BYTES);
+                const int nkt = x.nkt();
+                if constexpr (C::HALVES == 1) {
+                    bulk_g2s(dst, xbase + (size_t)x.kt0 * C::XTILE, (uint32_t)(nkt * C::XTILE), full_bar(xs));
+                } else {                                              // this pass's rows and sums of every k tile
+                    for (int kt = 0; kt < nkt; ++kt) {
+                        const uint8_t* tile = xbase + (size_t)(x.kt0 + kt) * (C::HALVES * C::XTILE);
+                        bulk_g2s(dst + kt * C::XTILE, tile + x.half * (C::ROWS * 128), C::ROWS * 128, full_bar(xs));
+                        for (int h = 0; h < C::GPT; ++h)
+                            bulk_g2s(dst + kt * C::XTILE + C::ROWS * (128 + 4 * h),
+                                     tile + C::HALVES * C::ROWS * (128 + 4 * h) + x.half * (C::ROWS * 4), C::ROWS * 4, full_bar(xs));
+                    }
+                }
+                if (++xs == STAGES) xs = 0;
+                x.next();
+                --ahead;
+            };
+            if (!multi) {
+                while (ahead < STAGES && w.valid()) {
+                    issue_w();
+                    if (ahead == 1) stamp(tr, 1);
+                }
+                if (!w.valid()) prefetch_next();
                 pdl_wait();
-                for (int e = 0; e < issued; ++e)
-                    bulk_g2s(smem_u32(stage0 + e * C::STAGE_BYTES + C::W_BYTES), a.xp + (size_t)early_kt0[e] * C::XTILE,
-                             (uint32_t)(early_nkt[e] * C::XTILE), full_bar(e));
             }
+            while (x.valid()) {
+                if (ahead == 0) issue_w();
+                issue_x();
+                if (!w.valid() && !prefetched) prefetch_next();
+            }
+            stamp(tr, 7);
         }
         return;
     }
+    if constexpr (C::REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     pdl_wait();                  // everything below reads or writes what other kernels produce or read
     if (threadIdx.x == 0) stamp(tr, 2);
     if (begin >= end) return;
@@ -278,11 +336,43 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
     uint32_t nib_mask = 0x000F000Fu, magic = 0x43004300u;
     asm volatile("" : "+r"(nib_mask), "+r"(magic));
     const uint32_t epoch = epoch_s;
+    // one accumulator unit (16 columns x 8 rows, a lane's 4 values) of column block `cb` to its destination
+    auto store_unit = [&](int cb, int prob, int half, int ti, int rb_pass, const float (&v)[4]) {
+        const int col0 = cb * kCols + (warp * T + ti) * 16 + g, rb = half * MB + rb_pass;
+        if (!MULTI && a.peer_bufs != nullptr) {
+            // a tensor-parallel rank's partial: straight into every rank's exchange buffer, self-signalling
+            const uint32_t want = *reinterpret_cast<const volatile uint32_t*>(a.peer_seq) + 1u;
+            const size_t base = (want & 1u) * a.peer_slot_bytes + (size_t)a.peer_rank * ((a.M + 1) / 2) * a.N * 16;
+#pragma unroll
+            for (int hsel = 0; hsel < 2; ++hsel) {
+                const int row = rb * 8 + 2 * t, col = col0 + hsel * 8;
+                if (row < a.M && col < a.N) {
+                    const size_t at = base + ((size_t)(row >> 1) * a.N + col) * 16;
+                    for (int peer = 0; peer < a.peer_world; ++peer)
+                        asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(a.peer_bufs[peer] + at),
+                                     "r"(__float_as_uint(v[2 * hsel])), "r"(want), "r"(__float_as_uint(v[2 * hsel + 1])), "r"(want) : "memory");
+                }
+            }
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = rb * 8 + 2 * t + (i & 1), col = col0 + (i >> 1) * 8;
+            if (row < a.M && col < a.N) {
+                const size_t at = (size_t)prob * a.y_stride + (size_t)row * a.N + col;
+                if (a.f32_out) reinterpret_cast<float*>(a.y)[at] = v[i];
+                else reinterpret_cast<__nv_bfloat16*>(a.y)[at] = f2bf(v[i]);
+            }
+        }
+    };
+    constexpr bool SHARED_SUM = MB > 1;
+    int parked = 0;                      // bit 2 * half: this range's first segment is parked, bit 2 * half + 1: its last
     float acc[T][MB][4];
     int s = 0;
     uint32_t phase = 0;
-    int it = begin;
-    while (it < end) {
+#pragma unroll 1
+    for (int half = 0; half < C::HALVES; ++half)
+    for (int it = begin; it < end;) {
         const int gb = it / SPB, pq = MULTI ? gb / CB : 0, cb = gb - pq * CB;
         const int prob = (MULTI && a.prob_sel) ? a.prob_sel[pq] : pq;
         const int cb_begin = gb * SPB, cb_end = cb_begin + SPB;
@@ -323,28 +413,47 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
                             sc[ti][h][1] = bf16_lo(p.y); bi[ti][h][1] = bf16_hi(p.y);
                         }
                     }
+                    // RP row blocks at a time: their chains of dependent products (25 cycles a step) run interleaved
+                    constexpr int RP = MB > 1 ? 2 : 1;
 #pragma unroll
-                    for (int rb = 0; rb < MB; ++rb) {
-                        const uint4 x0 = *reinterpret_cast<const uint4*>(xt + rb * 1024 + xlane);
-                        const uint4 x1 = *reinterpret_cast<const uint4*>(xt + rb * 1024 + (xlane ^ 64));
-                        const uint32_t xb[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                    for (int rb0 = 0; rb0 < MB; rb0 += RP) {
+                        uint32_t xb[RP][8];
+#pragma unroll
+                        for (int r = 0; r < RP; ++r) {
+                            const uint4 x0 = *reinterpret_cast<const uint4*>(xt + (rb0 + r) * 1024 + xlane);
+                            const uint4 x1 = *reinterpret_cast<const uint4*>(xt + (rb0 + r) * 1024 + (xlane ^ 64));
+                            xb[r][0] = x0.x; xb[r][1] = x0.y; xb[r][2] = x0.z; xb[r][3] = x0.w;
+                            xb[r][4] = x1.x; xb[r][5] = x1.y; xb[r][6] = x1.z; xb[r][7] = x1.w;
+                        }
                         constexpr int SPG = 4 / C::GPT;   // k-steps per group
 #pragma unroll
                         for (int h = 0; h < C::GPT; ++h) {
-                            const float2 xs = *reinterpret_cast<const float2*>(xsums + h * C::ROWS + rb * 8);
-                            const float i0 = -128.f * xs.x, i1 = -128.f * xs.y;
+                            float2 xs[RP];
+                            float p[RP][T][4];
 #pragma unroll
-                            for (int ti = 0; ti < T; ++ti) {
-                                float p[4] = {i0, i1, i0, i1};
+                            for (int r = 0; r < RP; ++r) xs[r] = *reinterpret_cast<const float2*>(xsums + h * C::ROWS + (rb0 + r) * 8);
 #pragma unroll
-                                for (int s4 = h * SPG; s4 < (h + 1) * SPG; ++s4)
-                                    mma_bf16_16816(p, af[ti][s4], xb[2 * s4], xb[2 * s4 + 1], p);
-                                float* ac = acc[ti][rb];
-                                ac[0] = __fmaf_rn(bi[ti][h][0], xs.x, __fmaf_rn(sc[ti][h][0], p[0], ac[0]));
-                                ac[1] = __fmaf_rn(bi[ti][h][0], xs.y, __fmaf_rn(sc[ti][h][0], p[1], ac[1]));
-                                ac[2] = __fmaf_rn(bi[ti][h][1], xs.x, __fmaf_rn(sc[ti][h][1], p[2], ac[2]));
-                                ac[3] = __fmaf_rn(bi[ti][h][1], xs.y, __fmaf_rn(sc[ti][h][1], p[3], ac[3]));
-                            }
+                            for (int s4 = h * SPG; s4 < (h + 1) * SPG; ++s4)
+#pragma unroll
+                                for (int r = 0; r < RP; ++r) {
+                                    const float i0 = -128.f * xs[r].x, i1 = -128.f * xs[r].y;
+                                    const float start[4] = {i0, i1, i0, i1};
+#pragma unroll
+                                    for (int ti = 0; ti < T; ++ti) {
+                                        if (s4 == h * SPG) mma_bf16_16816(p[r][ti], af[ti][s4], xb[r][2 * s4], xb[r][2 * s4 + 1], start);
+                                        else mma_bf16_16816(p[r][ti], af[ti][s4], xb[r][2 * s4], xb[r][2 * s4 + 1], p[r][ti]);
+                                    }
+                                }
+#pragma unroll
+                            for (int r = 0; r < RP; ++r)
+#pragma unroll
+                                for (int ti = 0; ti < T; ++ti) {
+                                    float* ac = acc[ti][rb0 + r];
+                                    ac[0] = __fmaf_rn(bi[ti][h][0], xs[r].x, __fmaf_rn(sc[ti][h][0], p[r][ti][0], ac[0]));
+                                    ac[1] = __fmaf_rn(bi[ti][h][0], xs[r].y, __fmaf_rn(sc[ti][h][0], p[r][ti][1], ac[1]));
+                                    ac[2] = __fmaf_rn(bi[ti][h][1], xs[r].x, __fmaf_rn(sc[ti][h][1], p[r][ti][2], ac[2]));
+                                    ac[3] = __fmaf_rn(bi[ti][h][1], xs[r].y, __fmaf_rn(sc[ti][h][1], p[r][ti][3], ac[3]));
+                                }
                         }
                     }
                 }
@@ -357,11 +466,26 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
 
         // ---- segment done ----
         if (tr != nullptr && threadIdx.x == 0 && seg_end == end) stamp(tr, 4);
-        if (seg_begin > cb_begin) {
+        if constexpr (SHARED_SUM) {
+            if (seg_begin > cb_begin || seg_end < cb_end) {
+                const int which = seg_begin > cb_begin ? 0 : 1;        // a worker's first and last segments may both be parts
+                float4* slot = reinterpret_cast<float4*>(a.slots + (size_t)(2 * blockIdx.x + which) * kSlotFloats) + half * (T * MB * NC);
+#pragma unroll
+                for (int ti = 0; ti < T; ++ti)
+#pragma unroll
+                    for (int rb = 0; rb < MB; ++rb)
+                        __stcg(slot + (ti * MB + rb) * NC + threadIdx.x, make_float4(acc[ti][rb][0], acc[ti][rb][1], acc[ti][rb][2], acc[ti][rb][3]));
+                __threadfence();
+                named_bar_sync(4, NC);
+                if (threadIdx.x == 0) st_release(a.flags + blockIdx.x * kFlagStride + 2 * half + which, epoch);
+                parked |= 1 << (2 * half + which);
+                continue;
+            }
+        } else if (seg_begin > cb_begin) {
             // a later segment of a block some earlier worker finishes: park it (always the first of this range)
             // as 16-byte packets {value, value, launch number, launch number}: a packet is stored whole, so a
             // reader that sees this launch's number in it has the values too. No fence, no flag.
-            float4* slot = reinterpret_cast<float4*>(a.slots + (size_t)blockIdx.x * (2 * kSlotFloats));
+            float4* slot = reinterpret_cast<float4*>(a.packets + (size_t)blockIdx.x * kPacketFloats);
             const float tagf = __uint_as_float(epoch);
 #pragma unroll
             for (int ti = 0; ti < T; ++ti)
@@ -373,7 +497,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
             if (tr != nullptr && threadIdx.x == 0) stamp(tr, 5);
             continue;
         }
-        if (seg_end < cb_end) {
+        if (!SHARED_SUM && seg_end < cb_end) {
             // the block's first segment: add the later ones, parked by the next workers, in worker order.
             // Up to four segments are waited for and fetched together (their latencies overlap) and then
             // added one by one, so the sum is the plain sequential one.
@@ -402,7 +526,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
 #pragma unroll
                         for (int j = 0; j < SB; ++j)
                             if (j < cnt) {
-                                const float4* slot = reinterpret_cast<const float4*>(a.slots + (size_t)who[j] * (2 * kSlotFloats));
+                                const float4* slot = reinterpret_cast<const float4*>(a.packets + (size_t)who[j] * kPacketFloats);
 #pragma unroll
                                 for (int u = 0; u < UB; ++u)
 #pragma unroll
@@ -467,44 +591,70 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
                 continue;
             }
         }
-        if (!MULTI && a.peer_bufs != nullptr) {
-            // a tensor-parallel rank's partial: straight into every rank's exchange buffer, self-signalling
-            const uint32_t want = *reinterpret_cast<const volatile uint32_t*>(a.peer_seq) + 1u;
-            const size_t base = (want & 1u) * a.peer_slot_bytes + (size_t)a.peer_rank * ((a.M + 1) / 2) * a.N * 16;
 #pragma unroll
-            for (int ti = 0; ti < T; ++ti) {
-                const int col0 = cb * kCols + (warp * T + ti) * 16 + g;
+        for (int ti = 0; ti < T; ++ti)
 #pragma unroll
-                for (int rb = 0; rb < MB; ++rb)
-#pragma unroll
-                    for (int hsel = 0; hsel < 2; ++hsel) {
-                        const int row = rb * 8 + 2 * t, col = col0 + hsel * 8;
-                        if (row < a.M && col < a.N) {
-                            const uint4 pkt = make_uint4(__float_as_uint(acc[ti][rb][2 * hsel]), want,
-                                                         __float_as_uint(acc[ti][rb][2 * hsel + 1]), want);
-                            const size_t at = base + ((size_t)(row >> 1) * a.N + col) * 16;
-                            for (int peer = 0; peer < a.peer_world; ++peer)
-                                asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(a.peer_bufs[peer] + at), "r"(pkt.x),
-                                             "r"(pkt.y), "r"(pkt.z), "r"(pkt.w) : "memory");
-                        }
-                    }
+            for (int rb = 0; rb < MB; ++rb) store_unit(cb, prob, half, ti, rb, acc[ti][rb]);
+    }
+    if constexpr (SHARED_SUM) {
+#pragma unroll 1
+        for (int part = 0; part < 2 * C::HALVES; ++part) {
+            if (!(parked >> part & 1)) continue;
+            const int half = part >> 1, which = part & 1;
+            // the cut block at this end of the range, and the workers that hold its segments, in k order
+            const int gb = (which == 0 ? begin : end - 1) / SPB, cb_begin = gb * SPB, cb_end = cb_begin + SPB;
+            int first = blockIdx.x, nseg = 0, mine = 0;
+            while (range_begin(first, total) > cb_begin) --first;
+            while (range_begin(first + 1, total) == cb_begin) ++first;     // a worker without work
+            int last = first;                                          // one past the block's last worker
+            for (; last < kWorkers && range_begin(last, total) < cb_end; ++last) {
+                if (last == (int)blockIdx.x) mine = nseg;
+                nseg += range_begin(last, total) < range_begin(last + 1, total);
             }
-            continue;
-        }
+            const bool sparse = nseg != last - first;                  // some of these workers have no work
+            bool ready = false;
+            for (int spin = 0; spin < (1 << 20) && !ready; ++spin) {
+                ready = true;
+                for (int w = first + lane; w < last; w += 32) {
+                    const bool idle = range_begin(w, total) == range_begin(w + 1, total);
+                    // the first segment is its worker's last part, every later one its worker's first part
+                    ready = ready && (idle || ld_acquire(a.flags + w * kFlagStride + 2 * half + (w == first ? 1 : 0)) == epoch);
+                }
+                ready = __all_sync(0xffffffffu, ready);
+            }
+            if (!ready) report(a.status, TF_ESTALL);
+            const float4* parts = reinterpret_cast<const float4*>(a.slots) + half * (T * MB * NC) + threadIdx.x;
+            constexpr size_t kSlot4 = kSlotFloats / 4;
+            // UB units' segments are fetched together: a fetch is an L2 round trip, whatever its size
+            constexpr int SB = 2, UN = T * MB, UB = UN >= 4 ? 4 : UN;
+#pragma unroll 1
+            for (int u0 = mine; u0 < UN; u0 += UB * nseg) {
+                float4 sum[UB];
 #pragma unroll
-        for (int ti = 0; ti < T; ++ti) {
-            const int col0 = cb * kCols + (warp * T + ti) * 16 + g;
+                for (int i = 0; i < UB; ++i)
+                    if (u0 + i * nseg < UN) sum[i] = __ldcg(parts + (2 * first + 1) * kSlot4 + (u0 + i * nseg) * NC);
+#pragma unroll 1
+                for (int w0 = first + 1; w0 < last; w0 += SB) {
+                    float4 v[SB][UB];
 #pragma unroll
-            for (int rb = 0; rb < MB; ++rb)
+                    for (int j = 0; j < SB; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = rb * 8 + 2 * t + (i & 1), col = col0 + (i >> 1) * 8;
-                    if (row < a.M && col < a.N) {
-                        const size_t at = (size_t)prob * a.y_stride + (size_t)row * a.N + col;
-                        if (a.f32_out) reinterpret_cast<float*>(a.y)[at] = acc[ti][rb][i];
-                        else reinterpret_cast<__nv_bfloat16*>(a.y)[at] = f2bf(acc[ti][rb][i]);
+                        for (int i = 0; i < UB; ++i)
+                            if (w0 + j < last && u0 + i * nseg < UN) v[j][i] = __ldcg(parts + 2 * (w0 + j) * kSlot4 + (u0 + i * nseg) * NC);
+#pragma unroll
+                    for (int j = 0; j < SB; ++j) {
+                        if (w0 + j >= last || (sparse && range_begin(w0 + j, total) == range_begin(w0 + j + 1, total))) continue;
+#pragma unroll
+                        for (int i = 0; i < UB; ++i) { sum[i].x += v[j][i].x; sum[i].y += v[j][i].y; sum[i].z += v[j][i].z; sum[i].w += v[j][i].w; }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < UB; ++i)
+                    if (u0 + i * nseg < UN) {
+                        const float r[4] = {sum[i].x, sum[i].y, sum[i].z, sum[i].w};
+                        store_unit(gb, 0, half, (u0 + i * nseg) / MB, (u0 + i * nseg) % MB, r);
+                    }
+            }
         }
     }
     if (threadIdx.x == 0) stamp(tr, 9);
@@ -512,7 +662,7 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) qmm_kernel(const Args a) 
 
 template <class C, bool MULTI = false>
 int launch(const Args& a, cudaStream_t stream) {
-    static_assert(C::SMEM <= (C::CTAS == 2 ? 113 : 227) * 1024, "stage ring does not fit shared memory");
+    static_assert(C::SMEM <= 227 * 1024, "stage ring does not fit shared memory");
     auto kern = qmm_kernel<C, MULTI>;
     // the opt-in is per device: keep one flag per device ordinal
     static bool configured[64] = {};
@@ -556,14 +706,18 @@ inline int prefetch_bytes() {
 
 template <int G>
 int dispatch(const Args& a, cudaStream_t stream) {
-    // up to 16 rows the kernel streams from HBM: a warp takes two column tiles, which share the activation
-    // loads; the wider buckets are bound by the tensor pipe and keep one tile a warp (their accumulators
-    // take the registers)
-    if (a.M <= 8) return launch<Cfg<G, 1, 4, 2, 1>>(a, stream);
-    if (a.M <= 16) return launch<Cfg<G, 2, 4, 2, 1>>(a, stream);
-    if (a.M <= 32) return launch<Cfg<G, 4, 4, 1, 1>>(a, stream);
-    if (a.M <= 64) return launch<Cfg<G, 8, 2, 1, 1>>(a, stream);
-    return launch<Cfg<G, 16, 2, 1, 1>>(a, stream);
+    // Eight consumer warps of two column tiles in every bucket. What bounds the loop above 8 rows is the sum of the warps'
+    // tensor, fma and integer instructions, not one of them: per SM, k tile and 8 rows 134 cycles of mma.sync (8.4 a
+    // sub-partition and m16n8k16, 545 TFLOP/s measured) and about 64 of fma, per k tile 270 of weight expansion. 16 warps
+    // of one tile, 16 warps of two tiles and half of the rows, and shorter stages measured the same or slower
+    // (17408 x 5120, 32 / 64 rows: 28.7 / 51.8 us; 31.1 / 53.2; 31.7 / 59.8).
+    // 128 rows take the 64-row pass twice (92 us, the weights' second pass comes out of L2): 128 accumulators a thread spill
+    // (104 us, and 143 us as 16 warps of one tile with one owner adding up the K segments).
+    if (a.M <= 8) return launch<Cfg<G, 1, 4, 2>>(a, stream);
+    if (a.M <= 16) return launch<Cfg<G, 2, 4, 2>>(a, stream);
+    if (a.M <= 32) return launch<Cfg<G, 4, 4, 2>>(a, stream);
+    if (a.M <= 64) return launch<Cfg<G, 8, 2, 2>>(a, stream);
+    return launch<Cfg<G, 8, 2, 2, 2>>(a, stream);
 }
 
 // ---- relayout kernels: one thread per output word / pair -----------------------------------------
@@ -636,6 +790,8 @@ __global__ void untile_kernel(const uint8_t* in, uint32_t* words, uint16_t* scal
 // sequential sum of 8, then a pairwise tree across the G/8 lanes of a group.
 template <int G>
 __global__ void pack_rows_kernel(const __nv_bfloat16* x, uint8_t* xp, float* xs_out, int M, int K) {
+    pdl_launch_dependents();     // the matmul behind it fills its ring with weights meanwhile
+    pdl_wait();
     const int Mp = tf_padded_rows(M);
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long chunks = (long long)Mp * (K >> 3);
@@ -699,7 +855,9 @@ int tf_qmm_next(const void* x_packed, const void* w_tiled, void* y, void* scratc
     a.w = static_cast<const uint8_t*>(w_tiled);
     a.y = y;
     a.epochs = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + tf::kEpochOffset);
+    a.flags = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + tf::kFlagOffset);
     a.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + TF_QMM_COUNTER_BYTES);
+    a.packets = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + tf::kPacketOffset);
     a.status = status;
     a.M = M; a.N = N; a.K = K;
     a.f32_out = (flags & TF_QMM_F32_OUT) ? 1 : 0;
@@ -760,7 +918,9 @@ int tf_qmm_grouped(const void* x_packed, const void* w_tiled, const int* prob_ex
     a.w = static_cast<const uint8_t*>(w_tiled);
     a.y = y;
     a.epochs = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + tf::kEpochOffset);
+    a.flags = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(scratch) + tf::kFlagOffset);
     a.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + TF_QMM_COUNTER_BYTES);
+    a.packets = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + tf::kPacketOffset);
     a.status = status;
     a.M = 8; a.N = N; a.K = K;
     a.f32_out = (flags & TF_QMM_F32_OUT) ? 1 : 0;
@@ -772,7 +932,7 @@ int tf_qmm_grouped(const void* x_packed, const void* w_tiled, const int* prob_ex
     a.xp_stride = (long long)tf_packed_bytes(8, K, group);
     a.y_stride = 8ll * N;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return group == 64 ? tf::launch<tf::Cfg<64, 1, 4, 2, 1>, true>(a, st) : tf::launch<tf::Cfg<32, 1, 4, 2, 1>, true>(a, st);
+    return group == 64 ? tf::launch<tf::Cfg<64, 1, 4, 2>, true>(a, st) : tf::launch<tf::Cfg<32, 1, 4, 2>, true>(a, st);
 }
 
 int tf_qmm_tile(const void* words, const void* scales, const void* biases, void* w_tiled, int N, int K, int group,
@@ -804,11 +964,10 @@ int tf_pack_rows(const void* x, void* x_packed, void* xs, int M, int K, int grou
     if (((uintptr_t)x | (uintptr_t)x_packed) & 15) return TF_EALIGN;
     const long long chunks = (long long)tf::tf_padded_rows(M) * (K / 8);
     const unsigned blocks = (unsigned)((chunks + 255) / 256);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    auto* xi = static_cast<const __nv_bfloat16*>(x);
-    if (group == 64) tf::pack_rows_kernel<64><<<blocks, 256, 0, st>>>(xi, static_cast<uint8_t*>(x_packed), static_cast<float*>(xs), M, K);
-    else tf::pack_rows_kernel<32><<<blocks, 256, 0, st>>>(xi, static_cast<uint8_t*>(x_packed), static_cast<float*>(xs), M, K);
-    return cudaGetLastError() == cudaSuccess ? TF_OK : TF_ECUDA;
+    void* args[] = {&x, &x_packed, &xs, &M, &K};
+    const void* fn = group == 64 ? (const void*)tf::pack_rows_kernel<64> : (const void*)tf::pack_rows_kernel<32>;
+    return tf::launch_pdl(fn, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream), args, 3) == cudaSuccess
+               ? TF_OK : (cudaGetLastError(), TF_ECUDA);
 }
 
 }  // extern "C"
