@@ -1,7 +1,7 @@
 // Gated-DeltaNet recurrence over the rows of each sequence's verify window, and the commit replay.
 //
 // Per (sequence, value head, value row) the fp32 state row S[0..127] (key dimension) stays in
-// registers across the window's rows, split over 4 lanes of 32 values each:
+// registers across the window's rows, split over 4 lanes of 32 values each (two value rows a thread):
 //     S    <- S * g
 //     mem   = S . k                      (fp32: per lane four 8-term fma chains combined pairwise, then a 4-lane xor tree)
 //     delta = (v - mem) * beta
@@ -12,7 +12,7 @@
 // serial one-row step would have produced, and row t of a window equals the t-th serial step.
 //
 // q and k of the rows being processed are staged as fp32 in shared memory, 8 rows at a time, and
-// shared by the 32 value rows a CTA owns.
+// shared by the 64 value rows a CTA owns.
 
 #include "common.cuh"
 
@@ -20,53 +20,113 @@ namespace tf {
 namespace {
 
 constexpr int kDk = 128;            // key head dim (state row length)
-constexpr int kRowsPerCta = 32;     // value rows per CTA: 4 lanes each -> 128 threads
+constexpr int kRowUnit = 32;        // value rows come in multiples of this
+constexpr int kRowsPerCta = 64;     // value rows per CTA of gdn_kernel: two a thread, 4 lanes each -> 128 threads
 constexpr int kTile = 8;            // window rows staged per pass
 
-// One window row applied to the 32 state values a lane holds (key elements 16*i + 4*j + e of one value row),
-// the same statements in the chain, replay and fused kernels: four partial dot products per lane (one per
-// element of the float4s, eight terms each, so the fma chains are short), combined pairwise, then the
-// 4-lane xor tree.
-template <bool OUT>
-__device__ __forceinline__ float gdn_row_step(float4 (&s)[8], const float* krow, const float* qrow, int j, float decay, float vval,
-                                              float beta) {
-    float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
+// ---- two fp32 lanes in one instruction: each half rounds as its scalar counterpart does ----
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// The 32 state values a lane holds of one value row: key elements 16*i + 4*j + e as pairs (e = 0,1) and (2,3).
+struct StateRow { ulonglong2 v[8]; };
+__device__ __forceinline__ void load_row(StateRow& s, const float* row, int j) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s.v[i] = reinterpret_cast<const ulonglong2*>(row)[i * 4 + j];
+}
+
+// One window row applied to the VR value rows a lane holds, the same statements in the chain, replay and fused
+// kernels: four partial dot products per value row and lane (one per element of the float4s, eight terms each,
+// so the fma chains are short), combined pairwise, then the 4-lane xor tree.
+//
+// A head's 128 x 128 state takes 65536 fp32 operations a window row, 512 cycles of an SM; one block alone spends about
+// 1050 (measured with clock64), the rest being the two dot products' reductions, which the next statement needs, and the loads of k
+// and q, which every lane of a value row's four repeats. Two value rows a thread share each load, k stays in registers
+// from the first dot product to the update, and the arithmetic runs on pairs (f32x2: the same rounding, half the
+// instructions): 128 warp loads of 16 bytes a head and row instead of 384.
+template <int VR, bool OUT>
+__device__ __forceinline__ void gdn_row_step(StateRow (&s)[VR], const float* krow, const float* qrow, int j, float decay, const float (&vval)[VR],
+                                             float beta, float (&out)[VR]) {
+    ulonglong2 kv[8];
+    f32x2 m01[VR], m23[VR];
+    const f32x2 decay2 = pack2(decay, decay);
+#pragma unroll
+    for (int r = 0; r < VR; ++r) m01[r] = m23[r] = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const float4 kv = *reinterpret_cast<const float4*>(krow + i * 16 + j * 4);
-        s[i].x *= decay; s[i].y *= decay; s[i].z *= decay; s[i].w *= decay;
-        m0 = __fmaf_rn(s[i].x, kv.x, m0);
-        m1 = __fmaf_rn(s[i].y, kv.y, m1);
-        m2 = __fmaf_rn(s[i].z, kv.z, m2);
-        m3 = __fmaf_rn(s[i].w, kv.w, m3);
-    }
-    float mem = (m0 + m1) + (m2 + m3);
-    mem += __shfl_xor_sync(0xffffffffu, mem, 1);
-    mem += __shfl_xor_sync(0xffffffffu, mem, 2);
-    const float delta = (vval - mem) * beta;
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+        kv[i] = *reinterpret_cast<const ulonglong2*>(krow + i * 16 + j * 4);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float4 kv = *reinterpret_cast<const float4*>(krow + i * 16 + j * 4);
-        s[i].x = __fmaf_rn(kv.x, delta, s[i].x);
-        s[i].y = __fmaf_rn(kv.y, delta, s[i].y);
-        s[i].z = __fmaf_rn(kv.z, delta, s[i].z);
-        s[i].w = __fmaf_rn(kv.w, delta, s[i].w);
-        if (OUT) {
-            const float4 qv = *reinterpret_cast<const float4*>(qrow + i * 16 + j * 4);
-            o0 = __fmaf_rn(s[i].x, qv.x, o0);
-            o1 = __fmaf_rn(s[i].y, qv.y, o1);
-            o2 = __fmaf_rn(s[i].z, qv.z, o2);
-            o3 = __fmaf_rn(s[i].w, qv.w, o3);
+        for (int r = 0; r < VR; ++r) {
+            s[r].v[i].x = mul2(s[r].v[i].x, decay2);
+            s[r].v[i].y = mul2(s[r].v[i].y, decay2);
+            m01[r] = fma2(s[r].v[i].x, kv[i].x, m01[r]);
+            m23[r] = fma2(s[r].v[i].y, kv[i].y, m23[r]);
         }
     }
-    float out = 0.f;
-    if (OUT) {
-        out = (o0 + o1) + (o2 + o3);
-        out += __shfl_xor_sync(0xffffffffu, out, 1);
-        out += __shfl_xor_sync(0xffffffffu, out, 2);
+    float mem[VR];
+#pragma unroll
+    for (int r = 0; r < VR; ++r) {
+        const float2 a = unpack2(m01[r]), b = unpack2(m23[r]);
+        mem[r] = (a.x + a.y) + (b.x + b.y);
     }
-    return out;
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1)
+#pragma unroll
+        for (int r = 0; r < VR; ++r) mem[r] += __shfl_xor_sync(0xffffffffu, mem[r], o);
+    f32x2 delta[VR], o01[VR], o23[VR];
+#pragma unroll
+    for (int r = 0; r < VR; ++r) {
+        const float d = (vval[r] - mem[r]) * beta;
+        delta[r] = pack2(d, d);
+        o01[r] = o23[r] = 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        ulonglong2 qv = make_ulonglong2(0, 0);
+        if (OUT) qv = *reinterpret_cast<const ulonglong2*>(qrow + i * 16 + j * 4);
+#pragma unroll
+        for (int r = 0; r < VR; ++r) {
+            s[r].v[i].x = fma2(kv[i].x, delta[r], s[r].v[i].x);
+            s[r].v[i].y = fma2(kv[i].y, delta[r], s[r].v[i].y);
+            if (OUT) {
+                o01[r] = fma2(s[r].v[i].x, qv.x, o01[r]);
+                o23[r] = fma2(s[r].v[i].y, qv.y, o23[r]);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < VR; ++r) {
+        out[r] = 0.f;
+        if (OUT) {
+            const float2 a = unpack2(o01[r]), b = unpack2(o23[r]);
+            out[r] = (a.x + a.y) + (b.x + b.y);
+        }
+    }
+    if (OUT) {
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1)
+#pragma unroll
+            for (int r = 0; r < VR; ++r) out[r] += __shfl_xor_sync(0xffffffffu, out[r], o);
+    }
 }
 
 struct GdnArgs {
@@ -87,16 +147,17 @@ struct GdnArgs {
 };
 
 template <bool OUT>
-__global__ void __launch_bounds__(kRowsPerCta * 4) gdn_kernel(const GdnArgs a) {
-    __shared__ float ks[kTile][kDk];
-    __shared__ float qs[OUT ? kTile : 1][kDk];
+__global__ void __launch_bounds__(kRowsPerCta * 2) gdn_kernel(const GdnArgs a) {
+    constexpr int THREADS = kRowsPerCta * 2, VR = 2;
+    __shared__ __align__(16) float ks[kTile][kDk];
+    __shared__ __align__(16) float qs[OUT ? kTile : 1][kDk];
     __shared__ float vs[kTile][kRowsPerCta];
     __shared__ float gs[kTile], bs[kTile];
     pdl_launch_dependents();
     pdl_wait();
     const int layer = blockIdx.z / a.S, seq = blockIdx.z % a.S, head = blockIdx.y;
-    const int tid = threadIdx.x, j = tid & 3, lr = tid >> 2;
-    const int dvrow = blockIdx.x * kRowsPerCta + lr;
+    const int tid = threadIdx.x, j = tid & 3, lr = tid >> 2;       // this thread's value rows: lr and lr + 32 of the CTA's
+    const int dv0 = blockIdx.x * kRowsPerCta;
     const int kh = head / (a.VH / a.KH);
     const int r0 = a.seq_start[seq];
     int n = a.seq_start[seq + 1] - r0;
@@ -106,21 +167,28 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gdn_kernel(const GdnArgs a) {
     const __nv_bfloat16* vp = a.v + layer * a.rec_v;
     const float* gp = a.g + layer * a.rec_g;
     const float* bp = a.beta + layer * a.rec_g;
-    const size_t srow = (size_t)layer * a.rec_state + (((size_t)seq * a.VH + head) * a.DV + dvrow) * kDk;
 
-    // lane j of a value row holds key elements 16*i + 4*j + e (i = 0..7, e = 0..3): float4 loads that coalesce
-    float4 s[8];
-    const bool live = dvrow < a.DV;
-    if (live) {
+    // lane j of a value row holds key elements 16*i + 4*j + e (i = 0..7, e = 0..3): 16-byte loads that coalesce
+    StateRow s[VR];
+    size_t srow[VR];
+    bool live[VR];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) s[i] = reinterpret_cast<const float4*>(a.state_in + srow)[i * 4 + j];
+    for (int x = 0; x < VR; ++x) {
+        const int dvrow = dv0 + lr + x * kRowUnit;
+        live[x] = dvrow < a.DV;
+        srow[x] = (size_t)layer * a.rec_state + (((size_t)seq * a.VH + head) * a.DV + dvrow) * kDk;
+        if (live[x]) load_row(s[x], a.state_in + srow[x], j);
+        else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[x].v[i] = make_ulonglong2(0, 0);
+        }
     }
 
     for (int t0 = 0; t0 < n; t0 += kTile) {
         const int rows = min(kTile, n - t0);
         __syncthreads();
-        // 16-byte loads: 8 bf16 values of a key/query row, or of a row's 32 values, per thread
-        for (int e = tid; e < rows * (kDk / 8); e += kRowsPerCta * 4) {
+        // 16-byte loads: 8 bf16 values of a key/query row, or of a row's 64 values, per thread
+        for (int e = tid; e < rows * (kDk / 8); e += THREADS) {
             const int r = e / (kDk / 8), d = (e % (kDk / 8)) * 8;
             const size_t at = ((size_t)(r0 + t0 + r) * a.KH + kh) * kDk + d;
             float f[8];
@@ -133,44 +201,41 @@ __global__ void __launch_bounds__(kRowsPerCta * 4) gdn_kernel(const GdnArgs a) {
                 for (int i = 0; i < 8; ++i) qs[r][d + i] = f[i];
             }
         }
-        if ((a.DV & 7) == 0) {
-            for (int e = tid; e < rows * (kRowsPerCta / 8); e += kRowsPerCta * 4) {
-                const int r = e / (kRowsPerCta / 8), c = (e % (kRowsPerCta / 8)) * 8;
-                const int dr = blockIdx.x * kRowsPerCta + c;
-                float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (dr < a.DV) unpack8(*reinterpret_cast<const uint4*>(vp + ((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dr), f);
+        for (int e = tid; e < rows * (kRowsPerCta / 8); e += THREADS) {
+            const int r = e / (kRowsPerCta / 8), c = (e % (kRowsPerCta / 8)) * 8;
+            float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (dv0 + c < a.DV) unpack8(*reinterpret_cast<const uint4*>(vp + ((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dv0 + c), f);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) vs[r][c + i] = f[i];
-            }
-        } else {
-            for (int e = tid; e < rows * kRowsPerCta; e += kRowsPerCta * 4) {
-                const int r = e / kRowsPerCta, c = e % kRowsPerCta;
-                const int dr = blockIdx.x * kRowsPerCta + c;
-                vs[r][c] = dr < a.DV ? bf2f(vp[((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dr]) : 0.f;
-            }
+            for (int i = 0; i < 8; ++i) vs[r][c + i] = f[i];
         }
         if (tid < rows) {
             gs[tid] = gp[(size_t)(r0 + t0 + tid) * a.VH + head];
             bs[tid] = bp[(size_t)(r0 + t0 + tid) * a.VH + head];
         }
         __syncthreads();
-        if (!live) continue;
         for (int r = 0; r < rows; ++r) {
-            const float out = gdn_row_step<OUT>(s, ks[r], qs[OUT ? r : 0], j, gs[r], vs[r][lr], bs[r]);
-            if (OUT && j == 0) a.y[((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dvrow] = f2bf(out);
+            const float v[VR] = {vs[r][lr], vs[r][lr + kRowUnit]};
+            float out[VR];
+            gdn_row_step<VR, OUT>(s, ks[r], qs[OUT ? r : 0], j, gs[r], v, bs[r], out);
+            if (OUT && j < VR && (j == 0 ? live[0] : live[1]))
+                a.y[((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dv0 + lr + j * kRowUnit] = f2bf(j == 0 ? out[0] : out[1]);
         }
     }
-    if (live && a.state_out != nullptr) {
+    if (a.state_out != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) reinterpret_cast<float4*>(a.state_out + srow)[i * 4 + j] = s[i];
+        for (int x = 0; x < VR; ++x)
+            if (live[x]) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) reinterpret_cast<ulonglong2*>(a.state_out + srow[x])[i * 4 + j] = s[x].v[i];
+            }
     }
 }
 
 // ---- the whole GDN mixer between its two projections, one launch ----------------------------------------
-// One CTA of 512 threads per (value head, sequence) does, for the sequence's window rows in passes of 8:
+// One CTA of 256 threads per (value head, sequence) does, for the sequence's window rows in passes of 8:
 //   1. the causal 4-tap conv + SiLU on the head's q, k and v channels, the RMS scale of q and k, the decay
-//      g and the write strength beta (one warp per (row, q | k | v), a lane's 4 channels: the statements of
-//      gdn_pre_kernel), into shared memory; k, v, g, beta also go to the record the commit replays;
+//      g and the write strength beta (one warp per row, a lane's 4 channels of q, k and v: the statements of
+//      gdn_pre_kernel), into shared memory, with SiLU(z) beside them; k, v, g, beta also go to the record the commit replays;
 //   2. the delta-rule recurrence over the pass's rows with the fp32 state row in registers (4 lanes x 32
 //      values per value row: the statements of gdn_kernel), y rounded to bf16 into shared memory;
 //   3. the gated RMSNorm of y with SiLU(z) (16 lanes per row: the statements of gated_norm_kernel) written
@@ -193,134 +258,136 @@ struct GdnFusedArgs {
     float eps;
 };
 
-template <int G>
-__global__ void __launch_bounds__(512) gdn_fused_kernel(const GdnFusedArgs a) {
-    __shared__ float ks[kTile][kDk], qs[kTile][kDk], vs[kTile][kDk], ys[kTile][kDk];
-    __shared__ float gs[kTile], bs[kTile];
+constexpr int kFusedThreads = 256;
+
+// CTAS: thread blocks an SM the registers are cut for. One block's time is a chain of phases (8 rows: conv 1.6 us,
+// recurrence 4.4, norm 1) whose latencies only another block fills; a grid of at most one block an SM is faster with all the
+// registers (32 heads x 8 rows: 9.5 against 11.7 us), a larger one with two blocks an SM (512 blocks: 33 against 36 us).
+// Before the pairs, the staged conv inputs and the gates up front: 10.2 us, 38.2 for 512 blocks, 135 (now 121) for a window of 128 rows.
+template <int G, int CTAS>
+__global__ void __launch_bounds__(kFusedThreads, CTAS) gdn_fused_kernel(const GdnFusedArgs a) {
+    __shared__ __align__(16) float ks[kTile][kDk], qs[kTile][kDk], vs[kTile][kDk], ys[kTile][kDk], zs[kTile][kDk];
+    __shared__ float gs[TF_QMM_MAX_ROWS], bs[TF_QMM_MAX_ROWS];
+    // conv inputs of a pass: its rows and the three before them, the head's q, k and v channels. The next pass's
+    // arrive (cp.async) while this pass's recurrence runs, so that a long window pays their trip once.
+    __shared__ __align__(16) __nv_bfloat16 raw[2][kTile + 3][3][kDk];
     pdl_launch_dependents();
     pdl_wait();
     const int head = blockIdx.x, seq = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int j = tid & 3, dvrow = tid >> 2;                       // recurrence roles: value row, quarter of the key axis
+    const int j = tid & 3, lr = tid >> 2;                          // recurrence roles: value rows lr and lr + 64, quarter of the key axis
     const int kh = head / (a.VH / a.KH);
     const int C = (2 * a.KH + a.VH) * 128;
     const int r0 = a.seq_start[seq], n = a.seq_start[seq + 1] - r0;
     const int Mp = tf_padded_rows(a.R), total = a.VH * 16;         // chunks of 8 in an output row
     // the last sequence's CTAs also zero the packed buffer's padding rows for their head
     if (seq == a.S - 1 && a.out_packed != nullptr) {
-        for (int e = tid; e < (Mp - a.R) * 16; e += 512)
+        for (int e = tid; e < (Mp - a.R) * 16; e += kFusedThreads)
             packed_store<G>(a.out_packed, Mp, a.R + e / 16, head * 16 + (e & 15), make_uint4(0, 0, 0, 0), 0.f);
     }
     if (n <= 0) return;
-    const size_t srow = (((size_t)seq * a.VH + head) * kDk + dvrow) * kDk;
-    float4 s[8];
+    // rows t0 .. t0 + rows + 2 of [conv_state (3 rows); window rows], 8 bytes a copy (the strides are multiples of four values)
+    auto stage = [&](int t0, int rows, int buf) {
+        for (int e = tid; e < (rows + 3) * 96; e += kFusedThreads) {
+            const int i = e / 96, part = (e % 96) >> 5, src = t0 + i;
+            const int ch0 = (part == 0 ? kh : part == 1 ? a.KH + kh : 2 * a.KH + head) * 128 + (e & 31) * 4;
+            const __nv_bfloat16* p = src < 3 ? a.conv_state + ((size_t)seq * 3 + src) * C + ch0 : a.qkv + (size_t)(r0 + src - 3) * a.qkv_stride + ch0;
+            cp_async8(smem_u32(&raw[buf][i][part][(e & 31) * 4]), p);
+        }
+        cp_async_commit();
+    };
+    stage(0, min(kTile, n), 0);
+    StateRow s[2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s[i] = reinterpret_cast<const float4*>(a.state_in + srow)[i * 4 + j];
+    for (int x = 0; x < 2; ++x) load_row(s[x], a.state_in + (((size_t)seq * a.VH + head) * kDk + lr + x * 64) * kDk, j);
+    // the window's gates, a thread a row
+    for (int t = tid; t < n; t += kFusedThreads) {
+        const size_t row = (size_t)(r0 + t);
+        const float av = bf2f(a.a_in[row * a.ab_stride + head]), bv = bf2f(a.b_in[row * a.ab_stride + head]);
+        const float ag = av + a.dt_bias[head];
+        const float sp = ag > 20.0f ? ag : logf(1.0f + expf(ag));
+        const float gv = expf(-expf(a.a_log[head]) * sp);
+        const float bvv = sigmoidf_(bv);
+        gs[t] = gv; bs[t] = bvv;
+        a.g_out[row * a.VH + head] = gv;
+        a.beta_out[row * a.VH + head] = bvv;
+    }
 
     for (int t0 = 0; t0 < n; t0 += kTile) {
-        const int rows = min(kTile, n - t0);
-        __syncthreads();
-        // ---- 1. conv + gates: warps 0..7 take q and k of row `warp`, warps 8..15 v and the gates of row
-        //         `warp - 8`; a warp's loads are all issued before the first use, so the pass costs one trip ----
-        {
-            const int r = warp & 7;
-            if (r < rows) {
-                const int row = r0 + t0 + r, idx = t0 + r;         // idx: the row's place in its sequence's chain
-                constexpr int NP = 2;
-                const int nparts = warp < 8 ? 2 : 1;
-                uint4 wq[NP][2];
-                uint2 xv[NP][4];
+        const int rows = min(kTile, n - t0), buf = (t0 / kTile) & 1;
+        // ---- 1. conv: warp r takes q, k and v of row r and its output gate z, side by side (each is one long dependent chain) ----
+        uint4 wq[3][2];
 #pragma unroll
-                for (int pi = 0; pi < NP; ++pi) {
-                    if (pi < nparts) {
-                        const int part = warp < 8 ? pi : 2;
-                        const int chead = part == 0 ? kh : part == 1 ? a.KH + kh : 2 * a.KH + head;
-                        const int ch0 = chead * 128 + lane * 4;
-                        const uint4* wp = reinterpret_cast<const uint4*>(a.conv_w + (size_t)ch0 * 4);
-                        wq[pi][0] = wp[0]; wq[pi][1] = wp[1];
+        for (int part = 0; part < 3; ++part) {
+            const int ch0 = (part == 0 ? kh : part == 1 ? a.KH + kh : 2 * a.KH + head) * 128 + lane * 4;
+            const uint4* wp = reinterpret_cast<const uint4*>(a.conv_w + (size_t)ch0 * 4);
+            wq[part][0] = wp[0]; wq[part][1] = wp[1];
+        }
+        uint2 zv = make_uint2(0, 0);                               // 8 bytes: the row stride is a multiple of four values (narrow shards)
+        if (warp < rows) zv = *reinterpret_cast<const uint2*>(a.z + (size_t)(r0 + t0 + warp) * a.z_stride + head * 128 + lane * 4);
+        cp_async_wait<0>();
+        __syncthreads();                                           // also: the last pass's readers of the shared rows are done
+        if (warp < rows) {
+            const int r = warp, row = r0 + t0 + r;
+            float c[4][4] = {{}, {}, {}, {bf16_lo(zv.x), bf16_hi(zv.x), bf16_lo(zv.y), bf16_hi(zv.y)}};
 #pragma unroll
-                        for (int tap = 0; tap < 4; ++tap) {
-                            const int src = idx + tap;             // index into [conv_state (3 rows); window rows]
-                            const __nv_bfloat16* p = src < 3 ? a.conv_state + ((size_t)seq * 3 + src) * C + ch0
-                                                             : a.qkv + (size_t)(row - idx + src - 3) * a.qkv_stride + ch0;
-                            xv[pi][tap] = *reinterpret_cast<const uint2*>(p);
-                        }
-                    }
-                }
-                float av = 0.f, bv = 0.f;
-                if (warp >= 8 && lane == 0) {
-                    av = bf2f(a.a_in[(size_t)row * a.ab_stride + head]);
-                    bv = bf2f(a.b_in[(size_t)row * a.ab_stride + head]);
+            for (int part = 0; part < 3; ++part) {
+                float wt[16];
+                {
+                    float lo[8], hi[8];
+                    unpack8(wq[part][0], lo);
+                    unpack8(wq[part][1], hi);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { wt[i] = lo[i]; wt[8 + i] = hi[i]; }
                 }
 #pragma unroll
-                for (int pi = 0; pi < NP; ++pi) {
-                    if (pi < nparts) {
-                        const int part = warp < 8 ? pi : 2;
-                        float wt[16];
-                        {
-                            float lo[8], hi[8];
-                            unpack8(wq[pi][0], lo);
-                            unpack8(wq[pi][1], hi);
+                for (int tap = 0; tap < 4; ++tap) {
+                    const uint2 xv = *reinterpret_cast<const uint2*>(&raw[buf][r + tap][part][lane * 4]);
+                    const float xf[4] = {bf16_lo(xv.x), bf16_hi(xv.x), bf16_lo(xv.y), bf16_hi(xv.y)};
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) { wt[i] = lo[i]; wt[8 + i] = hi[i]; }
-                        }
-                        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                        for (int tap = 0; tap < 4; ++tap) {
-                            const float xf[4] = {bf16_lo(xv[pi][tap].x), bf16_hi(xv[pi][tap].x), bf16_lo(xv[pi][tap].y), bf16_hi(xv[pi][tap].y)};
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) acc[i] = __fmaf_rn(xf[i], wt[i * 4 + tap], acc[i]);
-                        }
-                        float c[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) c[i] = round_bf16(acc[i] * sigmoidf_(acc[i]));
-                        if (part < 2) {
-                            float ss = 0.f;
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) ss += c[i] * c[i];
-                            const float inv = 1.0f / sqrtf(warp_sum(ss) / 128.0f + 1e-6f);
-                            const float scale = part == 0 ? 1.0f / 128.0f : 0.08838834764831845f;   // 1/dk, dk^-1/2
-                            const uint2 packed = make_uint2(pack_bf16(c[0] * inv * scale, c[1] * inv * scale),
-                                                            pack_bf16(c[2] * inv * scale, c[3] * inv * scale));
-                            float* dst = (part == 0 ? qs[r] : ks[r]) + lane * 4;
-                            dst[0] = bf16_lo(packed.x); dst[1] = bf16_hi(packed.x); dst[2] = bf16_lo(packed.y); dst[3] = bf16_hi(packed.y);
-                            // one of the value heads that share this key head keeps k for the commit
-                            if (part == 1 && head % (a.VH / a.KH) == 0)
-                                *reinterpret_cast<uint2*>(a.k_out + ((size_t)row * a.KH + kh) * 128 + lane * 4) = packed;
-                        } else {
-                            const uint2 packed = make_uint2(pack_bf16(c[0], c[1]), pack_bf16(c[2], c[3]));
-                            float* dst = vs[r] + lane * 4;
-                            dst[0] = c[0]; dst[1] = c[1]; dst[2] = c[2]; dst[3] = c[3];
-                            *reinterpret_cast<uint2*>(a.v_out + ((size_t)row * a.VH + head) * 128 + lane * 4) = packed;
-                            if (lane == 0) {
-                                const float ag = av + a.dt_bias[head];
-                                const float sp = ag > 20.0f ? ag : logf(1.0f + expf(ag));
-                                const float gv = expf(-expf(a.a_log[head]) * sp);
-                                const float bvv = sigmoidf_(bv);
-                                gs[r] = gv; bs[r] = bvv;
-                                a.g_out[(size_t)row * a.VH + head] = gv;
-                                a.beta_out[(size_t)row * a.VH + head] = bvv;
-                            }
-                        }
-                    }
+                    for (int i = 0; i < 4; ++i) c[part][i] = __fmaf_rn(xf[i], wt[i * 4 + tap], c[part][i]);
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {                         // SiLU of q, k, v (rounded) and of z
+                const float y = c[i >> 2][i & 3] * sigmoidf_(c[i >> 2][i & 3]);
+                c[i >> 2][i & 3] = i < 12 ? round_bf16(y) : y;
+            }
+            *reinterpret_cast<float4*>(zs[r] + lane * 4) = make_float4(c[3][0], c[3][1], c[3][2], c[3][3]);
+            float ss[2] = {0.f, 0.f};
+#pragma unroll
+            for (int part = 0; part < 2; ++part)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ss[part] += c[part][i] * c[part][i];
+#pragma unroll
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int part = 0; part < 2; ++part) ss[part] += __shfl_xor_sync(0xffffffffu, ss[part], o);
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                const float inv = 1.0f / sqrtf(ss[part] / 128.0f + 1e-6f);
+                const float scale = part == 0 ? 1.0f / 128.0f : 0.08838834764831845f;   // 1/dk, dk^-1/2
+                const uint2 packed = make_uint2(pack_bf16(c[part][0] * inv * scale, c[part][1] * inv * scale),
+                                                pack_bf16(c[part][2] * inv * scale, c[part][3] * inv * scale));
+                *reinterpret_cast<float4*>((part == 0 ? qs[r] : ks[r]) + lane * 4) =
+                    make_float4(bf16_lo(packed.x), bf16_hi(packed.x), bf16_lo(packed.y), bf16_hi(packed.y));
+                // one of the value heads that share this key head keeps k for the commit
+                if (part == 1 && head % (a.VH / a.KH) == 0)
+                    *reinterpret_cast<uint2*>(a.k_out + ((size_t)row * a.KH + kh) * 128 + lane * 4) = packed;
+            }
+            *reinterpret_cast<float4*>(vs[r] + lane * 4) = make_float4(c[2][0], c[2][1], c[2][2], c[2][3]);
+            *reinterpret_cast<uint2*>(a.v_out + ((size_t)row * a.VH + head) * 128 + lane * 4) = make_uint2(pack_bf16(c[2][0], c[2][1]), pack_bf16(c[2][2], c[2][3]));
         }
-        // the gated norm's z and weight, fetched now so that the trip hides behind the recurrence
-        uint4 z_pre = make_uint4(0, 0, 0, 0), w_pre = make_uint4(0, 0, 0, 0);
-        if (warp * 2 + (lane >> 4) < rows) {
-            const int row = r0 + t0 + warp * 2 + (lane >> 4), l16 = lane & 15;
-            // two 8-byte loads: a row stride that is only a multiple of four values (narrow tensor-parallel shards)
-            const uint2* zp = reinterpret_cast<const uint2*>(a.z + (size_t)row * a.z_stride + head * 128 + 8 * l16);
-            const uint2 z0 = zp[0], z1 = zp[1];
-            z_pre = make_uint4(z0.x, z0.y, z1.x, z1.y);
-            w_pre = reinterpret_cast<const uint4*>(a.norm_w)[l16];
-        }
+        // the next pass's conv inputs and the norm's weight: their trips hide behind the recurrence
+        if (t0 + kTile < n) stage(t0 + kTile, min(kTile, n - t0 - kTile), buf ^ 1);
+        const uint4 w_pre = reinterpret_cast<const uint4*>(a.norm_w)[lane & 15];
         __syncthreads();
         // ---- 2. recurrence over the pass's rows ----
         for (int r = 0; r < rows; ++r) {
-            const float out = gdn_row_step<true>(s, ks[r], qs[r], j, gs[r], vs[r][dvrow], bs[r]);
-            if (j == 0) ys[r][dvrow] = round_bf16(out);
+            const float v[2] = {vs[r][lr], vs[r][lr + 64]};
+            float out[2];
+            gdn_row_step<2, true>(s, ks[r], qs[r], j, gs[t0 + r], v, bs[t0 + r], out);
+            if (j < 2) ys[r][lr + j * 64] = round_bf16(j == 0 ? out[0] : out[1]);
         }
         __syncthreads();
         // ---- 3. gated norm + packing: 16 lanes per row, 8 values a lane ----
@@ -328,13 +395,16 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(const GdnFusedArgs a) {
             const int r = warp * 2 + (lane >> 4), l16 = lane & 15;
             const bool live = r < rows;
             const int row = r0 + t0 + (live ? r : 0);
-            float yv[8], zv[8], wv[8], o[8];
+            __align__(16) float yv[8], zv[8];
+            float wv[8], o[8];
             float ss = 0.f;
             uint4 ov = make_uint4(0, 0, 0, 0);
             if (live) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) yv[i] = ys[r][l16 * 8 + i];
-                unpack8(z_pre, zv);
+                for (int i = 0; i < 8; i += 4) {
+                    *reinterpret_cast<float4*>(yv + i) = *reinterpret_cast<const float4*>(ys[r] + l16 * 8 + i);
+                    *reinterpret_cast<float4*>(zv + i) = *reinterpret_cast<const float4*>(zs[r] + l16 * 8 + i);
+                }
                 unpack8(w_pre, wv);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) ss += yv[i] * yv[i];
@@ -344,7 +414,7 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(const GdnFusedArgs a) {
             if (live) {
                 const float inv = 1.0f / sqrtf(ss / 128.0f + a.eps);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = zv[i] * sigmoidf_(zv[i]) * (yv[i] * inv * wv[i]);
+                for (int i = 0; i < 8; ++i) o[i] = zv[i] * (yv[i] * inv * wv[i]);
                 ov = pack8(o);
             }
             const float gsum = group_sum8<G>(ov);
@@ -381,7 +451,7 @@ __global__ void conv_commit_kernel(const __nv_bfloat16* qkv, size_t qkv_stride, 
 }
 
 int check(int S, int layers, int KH, int VH, int DK, int DV) {
-    if (S < 1 || layers < 1 || KH < 1 || VH < 1 || VH % KH || DK != kDk || DV < 1 || DV % kRowsPerCta) return TF_EINVAL;
+    if (S < 1 || layers < 1 || KH < 1 || VH < 1 || VH % KH || DK != kDk || DV < 1 || DV % kRowUnit) return TF_EINVAL;
     if ((long long)S * layers > 65535) return TF_EINVAL;
     return TF_OK;
 }
@@ -405,7 +475,7 @@ int tf_gdn_chain(const void* q, const void* k, const void* v, const float* g, co
     a.KH = k_heads; a.VH = v_heads; a.DV = dv; a.S = n_seqs;
     void* args[] = {&a};
     dim3 grid((dv + tf::kRowsPerCta - 1) / tf::kRowsPerCta, v_heads, n_seqs);
-    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<true>, grid, dim3(tf::kRowsPerCta * 4), 0,
+    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<true>, grid, dim3(tf::kRowsPerCta * 2), 0,
                                    static_cast<cudaStream_t>(stream), args);
     if (e != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
@@ -433,8 +503,10 @@ int tf_gdn_fused(const void* qkv, size_t qkv_stride, const void* z, size_t z_str
     g.out_packed = static_cast<uint8_t*>(out_packed); g.out_rows = static_cast<__nv_bfloat16*>(out_rows);
     g.seq_start = seq_start; g.KH = k_heads; g.VH = v_heads; g.S = n_seqs; g.R = rows; g.group = group; g.eps = eps;
     void* args[] = {&g};
-    const void* fn = group == 64 ? (const void*)tf::gdn_fused_kernel<64> : (const void*)tf::gdn_fused_kernel<32>;
-    cudaError_t e = tf::launch_pdl(fn, dim3(v_heads, n_seqs), dim3(512), 0, static_cast<cudaStream_t>(stream), args);
+    const bool one = (long long)v_heads * n_seqs <= 148;         // a thread block an SM at most
+    const void* fn = group == 64 ? (one ? (const void*)tf::gdn_fused_kernel<64, 1> : (const void*)tf::gdn_fused_kernel<64, 2>)
+                                 : (one ? (const void*)tf::gdn_fused_kernel<32, 1> : (const void*)tf::gdn_fused_kernel<32, 2>);
+    cudaError_t e = tf::launch_pdl(fn, dim3(v_heads, n_seqs), dim3(tf::kFusedThreads), 0, static_cast<cudaStream_t>(stream), args);
     if (e != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
 }
@@ -454,7 +526,7 @@ int tf_gdn_replay(const void* k, const void* v, const float* g, const float* bet
     a.rec_q = rec_k_stride; a.rec_v = rec_v_stride; a.rec_g = rec_g_stride; a.rec_state = state_stride;
     void* args[] = {&a};
     dim3 grid((dv + tf::kRowsPerCta - 1) / tf::kRowsPerCta, v_heads, n_seqs * layers);
-    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<false>, grid, dim3(tf::kRowsPerCta * 4), 0,
+    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<false>, grid, dim3(tf::kRowsPerCta * 2), 0,
                                    static_cast<cudaStream_t>(stream), args);
     if (e != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
