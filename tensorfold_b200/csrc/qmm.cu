@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
                         }
                     }
                     // RP row blocks at a time: their chains of dependent products (25 cycles a step) run interleaved
-                    constexpr int RP = MB > 1 ? 2 : 1;
+                    constexpr int RP = MB == 4 ? 4 : MB > 1 ? 2 : 1;
 #pragma unroll
                     for (int rb0 = 0; rb0 < MB; rb0 += RP) {
                         uint32_t xb[RP][8];
