@@ -414,7 +414,8 @@ void tf_set_poll_limit(unsigned polls);
 /* ---- exact top-k and keyed sampling --------------------------------------------------------------
  * Each row's k largest bf16 logits (k <= 64), ordered by value descending then id ascending; ties at
  * the cut go to the smallest ids. idx int32 [rows, k], val fp32 [rows, k]. scratch: the slices'
- * candidates, tf_topk_scratch_bytes bytes, 8-byte aligned, no initialisation; two launches.
+ * candidates, tf_topk_scratch_bytes bytes (grows with rows, vocab and k: made for the largest call it serves
+ * the smaller ones), 8-byte aligned, no initialisation; two launches.
  * Replaces: engine/topk.py:20-146 (radix_topk, topk_rows). */
 size_t tf_topk_scratch_bytes(int rows, int vocab, int k);
 int tf_topk_rows(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, void* scratch,

@@ -19,6 +19,8 @@
 // (keys staged in shared memory, two atomic histograms with a match per key) took 111 us there, its merge 12 us and a
 // draw of one thread a row 19.5 us.
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace tf {
@@ -28,17 +30,17 @@ constexpr int kMaxK = 64;
 constexpr int kSliceThreads = 256, kChunks = 8;                       // a thread holds kChunks x 8 keys
 constexpr int kSliceMax = kSliceThreads * kChunks * 8 - 8;            // a slice off a 16-byte boundary takes one chunk more
 constexpr int kSliceMin = 4096;
-constexpr int kCand = 1024, kMaxSlices = 64, kMergeThreads = 128;
+constexpr int kCand = 1024, kMaxSlices = 64, kMergeThreads = 128, kSms = 148;
 
 // Slices are cut so that a few rows still give every SM a CTA (down to kSliceMin entries a slice, at most kMaxSlices),
 // many rows the longest slices: the result does not depend on the cut.
-__host__ __device__ inline int slice_len(int V, int rows) {
-    int slices = (V + kSliceMax - 1) / kSliceMax;
-    const int most = V / kSliceMin < kMaxSlices ? V / kSliceMin : kMaxSlices, want = (148 + rows - 1) / rows;
-    if (slices < want) slices = want < most ? want : (most > slices ? most : slices);
+inline int least_slices(int V) { return (V + kSliceMax - 1) / kSliceMax; }
+inline int most_slices(int V) { return std::min(V / kSliceMin, kMaxSlices); }
+inline int slice_len(int V, int rows) {
+    const int slices = std::max(least_slices(V), std::min(most_slices(V), (kSms + rows - 1) / rows));
     return (((V + slices - 1) / slices) + 7) & ~7;          // a multiple of 8 entries: slices of an aligned row are aligned
 }
-__host__ __device__ inline int slice_count(int V, int rows) { const int L = slice_len(V, rows); return (V + L - 1) / L; }
+inline int slice_count(int V, int rows) { const int L = slice_len(V, rows); return (V + L - 1) / L; }
 
 __device__ __forceinline__ uint32_t unsort_key(uint32_t k) { return (k & 0x8000u) ? (k & 0x7FFFu) : (~k & 0xFFFFu); }
 // two bf16 values -> two sortable keys: a negative value's bits are inverted, a positive one's sign bit is set
@@ -325,9 +327,14 @@ __global__ void sample_kernel(const int* idx, const float* val, int width, const
 
 extern "C" {
 
+// Fewer rows are cut into more slices, so a call's own lists, rows x slice_count, may be more than those of a call with more
+// rows (vocabulary 248320: 154 for 7 rows, 152 for 8). The size is a bound of them that grows with the rows, the
+// vocabulary and k, so that a workspace made for the largest call serves every smaller one.
 size_t tf_topk_scratch_bytes(int rows, int vocab, int k) {
     if (rows < 1 || vocab < 1 || k < 1 || k > tf::kMaxK) return 0;
-    return (size_t)rows * tf::slice_count(vocab, rows) * k * sizeof(unsigned long long);
+    const size_t least = (size_t)rows * tf::least_slices(vocab), most = (size_t)rows * tf::most_slices(vocab), wanted = (size_t)rows + tf::kSms - 1;
+    const size_t lists = std::max(least, std::min(most, wanted));
+    return lists * k * sizeof(unsigned long long);
 }
 
 static int topk(const void* x, size_t row_stride, int rows, int vocab, int k, int* idx, float* val, tf::Draw draw, void* scratch,
@@ -337,7 +344,7 @@ static int topk(const void* x, size_t row_stride, int rows, int vocab, int k, in
     if (reinterpret_cast<uintptr_t>(x) & 1) return TF_EALIGN;
     const int slices = tf::slice_count(vocab, rows);
     if (slices > tf::kMaxSlices) return TF_EINVAL;
-    if (!scratch || scratch_bytes < tf_topk_scratch_bytes(rows, vocab, k)) return TF_ESCRATCH;
+    if (!scratch || scratch_bytes < (size_t)rows * slices * k * sizeof(unsigned long long)) return TF_ESCRATCH;
     if (reinterpret_cast<uintptr_t>(scratch) & 7) return TF_EALIGN;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int len = tf::slice_len(vocab, rows), n = slices * k;
