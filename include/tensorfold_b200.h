@@ -412,7 +412,7 @@ int tf_norm_xs_peer(const void* x, const void* residual, const void* partials, i
 void tf_set_poll_limit(unsigned polls);
 
 /* ---- exact top-k and keyed sampling --------------------------------------------------------------
- * Each row's k largest bf16 logits (k <= 64), ordered by value descending then id ascending; ties at
+ * Each row's k largest bf16 logits (k <= 64, vocab <= 1048576), ordered by value descending then id ascending; ties at
  * the cut go to the smallest ids. idx int32 [rows, k], val fp32 [rows, k]. scratch: the slices'
  * candidates, tf_topk_scratch_bytes bytes (grows with rows, vocab and k: made for the largest call it serves
  * the smaller ones), 8-byte aligned, no initialisation; two launches.

@@ -34,7 +34,12 @@ constexpr int kCand = 1024, kMaxSlices = 64, kMergeThreads = 128, kSms = 148;
 
 // Slices are cut so that a few rows still give every SM a CTA (down to kSliceMin entries a slice, at most kMaxSlices),
 // many rows the longest slices: the result does not depend on the cut.
-inline int least_slices(int V) { return (V + kSliceMax - 1) / kSliceMax; }
+// A vocabulary too long for kMaxSlices slices of kSliceMax, up to kMaxSlices of all the keys that a CTA's threads hold (1048576
+// entries), still has kMaxSlices: where such a slice is off a 16-byte boundary it takes the exact route.
+inline int least_slices(int V) {
+    const int slices = (V + kSliceMax - 1) / kSliceMax;
+    return slices > kMaxSlices && V <= kMaxSlices * kSliceThreads * kChunks * 8 ? kMaxSlices : slices;
+}
 inline int most_slices(int V) { return std::min(V / kSliceMin, kMaxSlices); }
 inline int slice_len(int V, int rows) {
     const int slices = std::max(least_slices(V), std::min(most_slices(V), (kSms + rows - 1) / rows));
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(kSliceThreads, 4) topk_slice_kernel(const __nv
     }
     __syncthreads();
     int have = n_s;
-    if (have > kCand) {
+    if (have > kCand || chunks > kChunks * kSliceThreads) {
         __syncthreads();
         exact_slice(xr, n, v0, kk, c_s, &n_s, scan_s);
         have = kk;

@@ -33,3 +33,26 @@ def test_one_workspace_over_row_counts(lib, largest, vocab):
         _lib.check(lib.tf_topk_rows(x, vocab, rows, vocab, k, idx, val, room, size, _lib.stream()), f"{rows} rows")
         assert torch.equal(idx, want[0][:rows]) and torch.equal(val, want[1][:rows]), rows
     assert bool((room[size:] == 0x5A).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [1048063, 1048064, 1048065, 1048570, 1048576])
+@pytest.mark.parametrize("off", [0, 3])
+def test_the_largest_vocabularies(lib, vocab, off):
+    """Up to 64 slices of 16384 entries, on and off a 16-byte boundary (``off`` entries into a row)."""
+
+    from tensorfold_b200 import topk
+
+    rows, k = 2, 28
+    wide = torch.randn((rows, vocab + 8), generator=torch.Generator().manual_seed(vocab)).to(torch.bfloat16)
+    x = wide.cuda()[:, off:off + vocab]
+    idx, val = topk.topk_rows(x, k)
+    order = torch.sort(wide[:, off:off + vocab].float(), dim=1, descending=True, stable=True)
+    assert torch.equal(idx.cpu().long(), order.indices[:, :k]) and torch.equal(val.cpu(), order.values[:, :k])
+
+
+def test_a_longer_vocabulary_is_refused(lib):
+    from tensorfold_b200 import _lib
+
+    one = 256                                               # an address that a refused call does not read
+    assert lib.tf_topk_rows(one, 1048577, 1, 1048577, 1, one, one, one, 1 << 30, None) == _lib.TF_EINVAL
