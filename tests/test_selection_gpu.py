@@ -41,3 +41,22 @@ def test_fused_draw_equals_selection_then_draw(lib, vocab, top_k, top_p):
     fused = S.sample_rows(logits, positions, s)
     assert torch.equal(fused, S.sample_rows(logits, positions, s, top=S.top_candidates(logits, s)))
     assert np.array_equal(fused.cpu().numpy(), np.array(O.sample_rows(logits.float().cpu().numpy(), positions.cpu().numpy(), s)))
+
+
+@pytest.mark.parametrize("vocab,k", [(7, 7), (100, 64), (255, 33), (256, 32), (511, 64), (513, 64), (600, 28), (1025, 28), (1500, 64), (1848, 28), (2055, 64)])
+@pytest.mark.parametrize("off", [0, 5])
+def test_short_rows(lib, vocab, k, off):
+    """Slices whose entries leave some warps empty or partly filled, on and off a 16-byte boundary: random, in rising and falling
+    order, and with the largest values side by side at either end."""
+
+    from tensorfold_b200 import topk
+
+    gen = torch.Generator().manual_seed(vocab)
+    x = torch.randn((5, vocab + 8), generator=gen)
+    x[1], x[2] = x[1].sort().values, x[2].sort(descending=True).values
+    x[3, off:off + 9] += 50.0
+    x[4, off + vocab - 9:off + vocab] += 50.0
+    x = x.to(BF)
+    idx, val = topk.topk_rows(x.cuda()[:, off:off + vocab], k)
+    widx, wval = O.topk_rows(x[:, off:off + vocab].float().numpy(), k)
+    assert np.array_equal(idx.cpu().numpy(), widx) and np.array_equal(val.cpu().numpy(), wval)
