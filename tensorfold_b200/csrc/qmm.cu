@@ -88,8 +88,8 @@ struct Cfg {
 
 // Optional per-CTA timeline for profiling: when set (tf_qmm_set_trace), each launch writes eight
 // globaltimer stamps per CTA: 0 kernel entry, 1 first weight copy issued, 2 predecessor's memory visible
-// (griddepcontrol.wait passed), 3 consumers past their first full barrier, 4 main loop done, 5 last
-// segment parked or written, 6 ordered sum done, 7 producer's last copy issued.
+// (griddepcontrol.wait passed), 3 consumers past their first full barrier, 4 main loop done, 5 a cut block's
+// segment parked, 6 its ordered sum done, 7 producer's last copy issued, 9 end.
 __device__ unsigned long long* g_trace = nullptr;
 __device__ __forceinline__ unsigned long long now_ns() {
     unsigned long long t;
@@ -486,6 +486,7 @@ __global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
                 named_bar_sync(4, NC);
                 if (threadIdx.x == 0) st_release(a.flags + blockIdx.x * kFlagStride + 2 * half + which, epoch);
                 parked |= 1 << (2 * half + which);
+                if (threadIdx.x == 0) stamp(tr, 5);
                 continue;
             }
         } else if (seg_begin > cb_begin) {
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
             int o = blockIdx.x + 1;
             bool more = true;
             while (more) {
-                constexpr int SB = MB <= 2 ? 4 : 1;              // segments fetched together
+                constexpr int SB = 4;                            // segments fetched together
                 constexpr int UN = T * MB, UB = UN >= 4 ? 4 : UN;  // accumulator units (4 values each), units per fetch
                 int who[SB], cnt = 0;
                 for (; o < kWorkers && cnt < SB; ++o) {
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
             if (tr != nullptr && threadIdx.x == 0) stamp(tr, 6);
         }
         // a whole block, or a finished one: write the output
-        if constexpr (!MULTI && T == 2) {
+        if constexpr (!MULTI && MB == 1 && T == 2) {
             if (a.act_packed != nullptr) {
                 __shared__ float act_part[kWarps / 2][C::ROWS];
                 const int at = cb * (kWarps / 2) + warp;            // activation tile: 16 inputs of the down projection
@@ -665,6 +666,7 @@ __global__ void __launch_bounds__(C::THREADS, 1) qmm_kernel(const Args a) {
             };
             if (nseg >= T * MB) sum_units(std::integral_constant<int, 1>(), std::integral_constant<int, 8>());
             else sum_units(std::integral_constant<int, MB == 2 ? 2 : 4>(), std::integral_constant<int, MB == 2 ? 4 : 2>());
+            if (threadIdx.x == 0) stamp(tr, 6);
         }
     }
     if (threadIdx.x == 0) stamp(tr, 9);
@@ -720,7 +722,7 @@ int dispatch(const Args& a, cudaStream_t stream) {
     // tensor, fma and integer instructions, not one of them: per SM, k tile and 8 rows 134 cycles of mma.sync (8.4 a
     // sub-partition and m16n8k16, 545 TFLOP/s measured) and about 64 of fma, per k tile 270 of weight expansion. 16 warps
     // of one tile, 16 warps of two tiles and half of the rows, and shorter stages measured the same or slower
-    // (17408 x 5120, 32 / 64 rows: 28.7 / 51.8 us; 31.1 / 53.2; 31.7 / 59.8).
+    // (17408 x 5120, 32 / 64 rows: 27.4 / 51.8 us; 34.1 / 53.2 with 16 warps of one tile; 31.7 / 59.8).
     // 128 rows take the 64-row pass twice (92 us, the weights' second pass comes out of L2): 128 accumulators a thread spill
     // (104 us, and 143 us as 16 warps of one tile with one owner adding up the K segments).
     if (a.M <= 8) return launch<Cfg<G, 1, 4, 2>>(a, stream);

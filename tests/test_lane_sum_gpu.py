@@ -28,3 +28,29 @@ def test_any_split_has_the_bits_of_single_rows(lib, n, k):
     assert_close(y.to(torch.bfloat16), O.qmm(x.cpu(), q.words, q.scales, q.biases, 64), f"{n}x{k}")
     torch.cuda.synchronize()
     _lib.status(y.device).raise_if_set()
+
+
+@pytest.mark.parametrize("rows", [8, 16, 64, 128])
+def test_timeline_stamps_of_cut_blocks(lib, rows):
+    """Workers that park a segment stamp it (5), and those that add parked segments stamp the sum's end (6), in every bucket."""
+
+    from tensorfold_b200 import _lib, lane_qmm, synthetic
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    w = synthetic.random_q4(gen, 5120, 4096, 64, "cuda")
+    x = lane_qmm.pack_rows(torch.randn((rows, 4096), generator=gen, device="cuda").to(torch.bfloat16), 64)
+    stamps = torch.zeros(148 + 512 * 148 * 16, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(lib.tf_qmm_set_trace(stamps), "trace")
+    try:
+        lane_qmm.lane_matmul(x, w)
+        torch.cuda.synchronize()
+    finally:
+        _lib.check(lib.tf_qmm_set_trace(None), "trace off")
+    s = stamps[148:148 + 148 * 16].reshape(148, 16).cpu()
+    done, parked, summed, end = s[:, 4], s[:, 5], s[:, 6], s[:, 9]
+    assert bool((done > 0).all()) and bool((end >= done).all())
+    assert int((parked > 0).sum()) >= 128 and int((summed > 0).sum()) >= 20      # 20 column blocks, all of them cut
+    at = (parked > 0) & (summed > 0)
+    if rows > 8:                                             # every worker that parks also adds
+        assert bool((summed[at] >= parked[at]).all()) and int(at.sum()) == int((parked > 0).sum())
