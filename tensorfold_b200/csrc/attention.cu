@@ -25,7 +25,7 @@
 namespace tf {
 namespace {
 
-constexpr int kTileKeys = 64, kPage = 16, kQRows = 64, kAttnWarps = 4;
+constexpr int kTileKeys = 64, kPage = 16, kQRows = 64, kAttnWarps = 4, kSms = 148;
 // chunk c covers keys [chunk_begin(c), chunk_begin(c + 1)): a function of the absolute position only
 constexpr int kSmallKeys = 128, kSmallChunks = 64, kMidKeys = 512, kMidChunks = 112, kBigKeys = 2048;
 constexpr int kSmallEnd = kSmallKeys * kSmallChunks, kMidEnd = kSmallEnd + kMidKeys * kMidChunks;   // 8192, 65536
@@ -76,13 +76,12 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 template <int D>
 __device__ __forceinline__ uint32_t swz(int r, int c) { return (uint32_t)(r * (D * 2) + (((c & ~7) | ((c ^ r) & 7)) << 4)); }
 
-// What bounds it is latency: a tile is 64 KB (D = 256) that three or four warps multiply between two waits. NB = 1: K and V
-// have one buffer each, the copy of the next K runs behind the softmax and P V, that of the next V behind the next Q K^T; the block
-// takes 96 KB, so two blocks an SM fill each other's waits (16 sequences x 4096 keys x 8 rows: 183 -> 146 us a layer).
-// NB = 2: two buffers, one block an SM, for a grid that leaves no SM two blocks: both tiles of a 128-key chunk are under way at once
-// (1 sequence x 4096 keys: 27 us, 32 with one buffer).
+// What bounds it is latency: a tile is 64 KB (D = 256) that three or four warps multiply between two waits. NB = 2: two K and two V
+// buffers, one block an SM: both tiles of a 128-key chunk are under way at once (1 sequence x 4096 keys x 8 rows: 18.7 us). NB = 1: one
+// buffer each, the copy of the next K runs behind the softmax and P V, that of the next V behind the next Q K^T; the block
+// takes 96 KB, and two of them fill each other's waits on an SM (16 sequences x 4096 keys x 8 rows: 182 -> 146 us a layer).
 template <int D, int NB>
-__global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(kAttnWarps * 32, D == 256 ? 3 - NB : 1) attn_chunk_kernel(const AttnArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int ROWB = D * 2, TILEB = kTileKeys * ROWB, CPR = D / 8;       // chunks of 16 B per row
     uint8_t* q_s = smem;                       // [64][D]
@@ -109,10 +108,10 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
     }
     const int* pt = a.page_table + (size_t)seq * a.max_pages;
     // A tile is four pages of 16 keys; warp w copies page w: the page number is looked up once, then
-    // every lane streams its own 16-byte column of the page's rows, so the per-copy address
-    // work is an add. Rows at or past the committed length come from the window's own K/V rows, rows
+    // every lane streams its own 16-byte column of the page's rows (K to k_dst and V to v_dst, either may be null), so the per-copy
+    // address work is an add. Rows at or past the committed length come from the window's own K/V rows, rows
     // past the last key are zero-filled.
-    auto load_tile = [&](const __nv_bfloat16* fresh, const __nv_bfloat16* pages, uint8_t* dst_s, int tile) {
+    auto load_tile = [&](int tile, uint8_t* k_dst, uint8_t* v_dst) {
         constexpr int RPI = 32 / CPR > 0 ? 32 / CPR : 1;      // rows a warp covers per step (1 for D = 256, 2 for D = 128)
         const int base = key0 + tile * kTileKeys + warp * kPage;
         const int c = lane % CPR, rsub = lane / CPR;
@@ -122,25 +121,18 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
         for (int rr = 0; rr < kPage; rr += RPI) {
             const int r = rr + rsub, p = base + r;
             const bool ok = p < L + n;
-            const __nv_bfloat16* src = fresh;
-            if (ok) src = p < L ? pages + page_off + (size_t)r * D + c * 8 : fresh + ((size_t)(r0 + p - L) * a.HK + kvh) * D + c * 8;
-            cp_async16_zfill(smem_u32(dst_s + swz<D>(warp * kPage + r, c)), src, ok);
+            size_t off = 0;
+            const __nv_bfloat16 *ksrc = a.k_new, *vsrc = a.v_new;
+            if (ok) {
+                if (p < L) { off = page_off + (size_t)r * D + c * 8; ksrc = a.k_pages; vsrc = a.v_pages; }
+                else off = ((size_t)(r0 + p - L) * a.HK + kvh) * D + c * 8;
+            }
+            const uint32_t dst = swz<D>(warp * kPage + r, c);
+            if (k_dst != nullptr) cp_async16_zfill(smem_u32(k_dst + dst), ksrc + off, ok);
+            if (v_dst != nullptr) cp_async16_zfill(smem_u32(v_dst + dst), vsrc + off, ok);
         }
     };
     const int ntiles = min(chunk_keys / kTileKeys, (L + n - key0 + kTileKeys - 1) / kTileKeys);
-    // one commit group a K or V tile, in order (an empty one past the last): tile t's K has 2 NB - 1 groups behind it when it is waited for
-    auto load_k = [&](int tile) {
-        if (tile < ntiles) load_tile(a.k_new, a.k_pages, k_s + (tile % NB) * TILEB, tile);
-        cp_async_commit();
-    };
-    auto load_v = [&](int tile) {
-        if (tile < ntiles) load_tile(a.v_new, a.v_pages, v_s + (tile % NB) * TILEB, tile);
-        cp_async_commit();
-    };
-    for (int tile = 0; tile < NB; ++tile) {
-        load_k(tile);
-        load_v(tile);
-    }
 
     // this warp's 16 query rows; lane holds rows g and g+8 of them
     const int qrow_lo = q0 + warp * 16 + g, qrow_hi = qrow_lo + 8;
@@ -153,15 +145,30 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
     for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
 
+    // NB = 2: a commit group a tile. NB = 1: one a K or V tile, in order (an empty one past the last). Either way one group is behind
+    // the one that is waited for.
+    load_tile(0, k_s, NB == 2 ? v_s : nullptr);
+    cp_async_commit();
+    if constexpr (NB == 1) {
+        load_tile(0, nullptr, v_s);
+        cp_async_commit();
+    }
     for (int tile = 0; tile < ntiles; ++tile) {
-        cp_async_wait<2 * NB - 1>();                       // K of this tile; its V may still be on the way
+        const int buf = NB == 2 ? tile & 1 : 0;
+        const bool more = tile + 1 < ntiles;
+        if constexpr (NB == 2) {
+            if (more) load_tile(tile + 1, k_s + (buf ^ 1) * TILEB, v_s + (buf ^ 1) * TILEB);
+            cp_async_commit();
+        }
+        cp_async_wait<1>();                                // K of this tile, with NB = 2 its V too
         __syncthreads();
         float s[8][4];
+        uint32_t pf[8][2];
         if (warp_live) {
             // ---- S = Q K^T for 16 rows x 64 keys ----
 #pragma unroll
             for (int i = 0; i < 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
-            const uint32_t kb = smem_u32(k_s + (tile % NB) * TILEB), qb = smem_u32(q_s);
+            const uint32_t kb = smem_u32(k_s + buf * TILEB), qb = smem_u32(q_s);
 #pragma unroll 4
             for (int ks = 0; ks < D / 16; ++ks) {
                 uint32_t af[4];
@@ -175,9 +182,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
                 }
             }
         }
-        if (tile + NB < ntiles) __syncthreads();           // every warp is done with K
-        load_k(tile + NB);
-        uint32_t pf[8][2];
+        if constexpr (NB == 1) {
+            if (more) {
+                __syncthreads();                           // every warp is done with K
+                load_tile(tile + 1, k_s, nullptr);
+            }
+            cp_async_commit();
+        }
         if (warp_live) {
             // ---- mask, online softmax (log2 domain) ----
             const int pbase = key0 + tile * kTileKeys + 2 * t;
@@ -217,11 +228,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
 #pragma unroll
             for (int i = 0; i < D / 8; ++i) { o[i][0] *= al_lo; o[i][1] *= al_lo; o[i][2] *= al_hi; o[i][3] *= al_hi; }
         }
-        cp_async_wait<2 * NB - 1>();                       // V of this tile
-        __syncthreads();
+        if constexpr (NB == 1) {
+            cp_async_wait<1>();                            // V of this tile
+            __syncthreads();
+        }
         if (warp_live) {
             // ---- O += P V ----
-            const uint32_t vb = smem_u32(v_s + (tile % NB) * TILEB);
+            const uint32_t vb = smem_u32(v_s + buf * TILEB);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {               // 16 keys a step
                 const uint32_t pa[4] = {pf[2 * kk][0], pf[2 * kk][1], pf[2 * kk + 1][0], pf[2 * kk + 1][1]};
@@ -234,8 +247,15 @@ __global__ void __launch_bounds__(kAttnWarps * 32, 3 - NB) attn_chunk_kernel(con
                 }
             }
         }
-        if (tile + NB < ntiles) __syncthreads();           // every warp is done with V
-        load_v(tile + NB);
+        if constexpr (NB == 2) {
+            __syncthreads();                               // every warp is done with this tile's buffers
+        } else {
+            if (more) {
+                __syncthreads();                           // every warp is done with V
+                load_tile(tile + 1, nullptr, v_s);
+            }
+            cp_async_commit();
+        }
     }
     cp_async_wait<0>();
     if (!warp_live) return;
@@ -420,22 +440,28 @@ struct GateArgs {
 
 template <int D>
 int run(const AttnArgs& a, int n_seqs, int max_chunks, const int* row_nkeys, void* out, cudaStream_t st, const GateArgs& ga = GateArgs()) {
-    // without a second block for any SM the buffers are the block's own (live blocks are at most the grid's)
-    const bool alone = (long long)max_chunks * a.HK * n_seqs * a.qgroups <= 148;
-    const void* kern = alone ? (const void*)attn_chunk_kernel<D, 2> : (const void*)attn_chunk_kernel<D, 1>;
-    const size_t smem = (size_t)(kQRows + (alone ? 4 : 2) * kTileKeys) * D * 2;
+    // Two buffers where every block of the grid has an SM of its own, and wherever it may have: the grid covers the capacity, the
+    // blocks that hold keys are often far fewer (1 sequence, 4 KV heads, 1024 / 4096 / 16384 keys in a capacity of 32768: 15.1 / 20.5 / 62 us;
+    // 19.2 / 23.0 / 71 with one; between 5000 and 8192 keys one is the faster, 28 against 31). From 16 (sequence, KV head, query group)
+    // columns on, one buffer is the faster at every length (4 x 4 columns, 1024 / 8192 keys: 22 / 77 us against 23 / 93; 16 x 4,
+    // 200 / 4096: 27 / 146 against 30 / 182).
+    // At D = 128 registers allow two blocks an SM either way.
+    const long long columns = (long long)a.HK * n_seqs * a.qgroups;
+    const bool two = D == 128 || columns < 16 || max_chunks * columns <= kSms;
+    const void* kern = two ? (const void*)attn_chunk_kernel<D, 2> : (const void*)attn_chunk_kernel<D, D == 128 ? 2 : 1>;
+    const auto bytes = [](int buffers) { return (kQRows + 2 * buffers * kTileKeys) * D * 2; };
     static bool configured[64] = {};       // the opt-in is per device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return TF_ECUDA; }
     if (!configured[dev]) {
-        if (cudaFuncSetAttribute(attn_chunk_kernel<D, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (kQRows + 2 * kTileKeys) * D * 2) != cudaSuccess ||
-            cudaFuncSetAttribute(attn_chunk_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (kQRows + 4 * kTileKeys) * D * 2) != cudaSuccess)
+        if (cudaFuncSetAttribute(attn_chunk_kernel<D, D == 128 ? 2 : 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(D == 128 ? 2 : 1)) != cudaSuccess ||
+            cudaFuncSetAttribute(attn_chunk_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes(2)) != cudaSuccess)
             return TF_ECUDA;
         configured[dev] = true;
     }
     AttnArgs args = a;
     void* p1[] = {&args};
-    if (launch_pdl(kern, dim3(max_chunks, a.HK, n_seqs * a.qgroups), dim3(kAttnWarps * 32), smem,
+    if (launch_pdl(kern, dim3(max_chunks, a.HK, n_seqs * a.qgroups), dim3(kAttnWarps * 32), bytes(two ? 2 : 1),
                    st, p1) != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     MergeArgs m;
     m.part_o = a.part_o; m.part_m = a.part_m; m.part_l = a.part_l; m.row_nkeys = row_nkeys;
