@@ -1,7 +1,7 @@
 // Gated-DeltaNet recurrence over the rows of each sequence's verify window, and the commit replay.
 //
 // Per (sequence, value head, value row) the fp32 state row S[0..127] (key dimension) stays in
-// registers across the window's rows, split over 4 lanes of 32 values each (two value rows a thread):
+// registers across the window's rows, split over 4 lanes of 32 values each (one or two value rows a thread):
 //     S    <- S * g
 //     mem   = S . k                      (fp32: per lane four 8-term fma chains combined pairwise, then a 4-lane xor tree)
 //     delta = (v - mem) * beta
@@ -12,7 +12,7 @@
 // serial one-row step would have produced, and row t of a window equals the t-th serial step.
 //
 // q and k of the rows being processed are staged as fp32 in shared memory, 8 rows at a time, and
-// shared by the 64 value rows a CTA owns.
+// shared by the 32 or 64 value rows a CTA owns.
 
 #include "common.cuh"
 
@@ -21,7 +21,7 @@ namespace {
 
 constexpr int kDk = 128;            // key head dim (state row length)
 constexpr int kRowUnit = 32;        // value rows come in multiples of this
-constexpr int kRowsPerCta = 64;     // value rows per CTA of gdn_kernel: two a thread, 4 lanes each -> 128 threads
+constexpr int kGdnThreads = 128;    // threads per CTA of gdn_kernel: 4 lanes a value row, VR rows a thread -> 32 VR value rows
 constexpr int kTile = 8;            // window rows staged per pass
 
 // ---- two fp32 lanes in one instruction: each half rounds as its scalar counterpart does ----
@@ -146,9 +146,9 @@ struct GdnArgs {
     int S;
 };
 
-template <bool OUT>
-__global__ void __launch_bounds__(kRowsPerCta * 2) gdn_kernel(const GdnArgs a) {
-    constexpr int THREADS = kRowsPerCta * 2, VR = 2;
+template <bool OUT, int VR, int CTAS>
+__global__ void __launch_bounds__(kGdnThreads, CTAS) gdn_kernel(const GdnArgs a) {
+    constexpr int THREADS = kGdnThreads, kRowsPerCta = kRowUnit * VR;
     __shared__ __align__(16) float ks[kTile][kDk];
     __shared__ __align__(16) float qs[OUT ? kTile : 1][kDk];
     __shared__ float vs[kTile][kRowsPerCta];
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kRowsPerCta * 2) gdn_kernel(const GdnArgs a) {
     pdl_launch_dependents();
     pdl_wait();
     const int layer = blockIdx.z / a.S, seq = blockIdx.z % a.S, head = blockIdx.y;
-    const int tid = threadIdx.x, j = tid & 3, lr = tid >> 2;       // this thread's value rows: lr and lr + 32 of the CTA's
+    const int tid = threadIdx.x, j = tid & 3, lr = tid >> 2;       // this thread's value rows: lr (and lr + 32) of the CTA's
     const int dv0 = blockIdx.x * kRowsPerCta;
     const int kh = head / (a.VH / a.KH);
     const int r0 = a.seq_start[seq];
@@ -214,11 +214,12 @@ __global__ void __launch_bounds__(kRowsPerCta * 2) gdn_kernel(const GdnArgs a) {
         }
         __syncthreads();
         for (int r = 0; r < rows; ++r) {
-            const float v[VR] = {vs[r][lr], vs[r][lr + kRowUnit]};
-            float out[VR];
+            float v[VR], out[VR];
+#pragma unroll
+            for (int x = 0; x < VR; ++x) v[x] = vs[r][lr + x * kRowUnit];
             gdn_row_step<VR, OUT>(s, ks[r], qs[OUT ? r : 0], j, gs[r], v, bs[r], out);
-            if (OUT && j < VR && (j == 0 ? live[0] : live[1]))
-                a.y[((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dv0 + lr + j * kRowUnit] = f2bf(j == 0 ? out[0] : out[1]);
+            if (OUT && j < VR && (j == 0 ? live[0] : live[VR - 1]))
+                a.y[((size_t)(r0 + t0 + r) * a.VH + head) * a.DV + dv0 + lr + j * kRowUnit] = f2bf(j == 0 ? out[0] : out[VR - 1]);
         }
     }
     if (a.state_out != nullptr) {
@@ -450,6 +451,21 @@ __global__ void conv_commit_kernel(const __nv_bfloat16* qkv, size_t qkv_stride, 
     for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(st + (size_t)i * C) = out[i];
 }
 
+// A value row a thread where its 32-row blocks find an SM each: a window row is then a chain of half the arithmetic (replay, 32 heads x 1 row:
+// 3.4 -> 2.9 us, 4 heads x 8 rows 4.4 -> 3.7; chain, 4 heads x 8 rows 5.1 -> 4.3; the chain's 64-row blocks hide theirs from about 100 small
+// blocks on: 32 heads x 8 rows 5.4 against 5.8). Larger grids take two rows a thread, for the shared loads of k and q; a replay of many
+// waves with the registers of four blocks an SM (12 layers x 16 x 8 rows: 185 against 204 us), one of few with those of three
+// (6 layers x 1 x 8 rows: 7.7 against 9.5).
+template <bool OUT>
+cudaError_t launch_gdn(GdnArgs a, int windows, void* stream) {
+    const long long blocks = (long long)(a.DV / kRowUnit) * a.VH * windows;
+    const bool one = blocks <= (OUT ? 100 : 148);
+    const void* fn = one ? (const void*)gdn_kernel<OUT, 1, 4> : blocks > 888 ? (const void*)gdn_kernel<OUT, 2, 4> : (const void*)gdn_kernel<OUT, 2, OUT ? 4 : 3>;
+    void* args[] = {&a};
+    const int per = kRowUnit * (one ? 1 : 2);
+    return launch_pdl(fn, dim3((a.DV + per - 1) / per, a.VH, windows), dim3(kGdnThreads), 0, static_cast<cudaStream_t>(stream), args);
+}
+
 int check(int S, int layers, int KH, int VH, int DK, int DV) {
     if (S < 1 || layers < 1 || KH < 1 || VH < 1 || VH % KH || DK != kDk || DV < 1 || DV % kRowUnit) return TF_EINVAL;
     if ((long long)S * layers > 65535) return TF_EINVAL;
@@ -473,10 +489,7 @@ int tf_gdn_chain(const void* q, const void* k, const void* v, const float* g, co
     a.state_in = state; a.state_out = state_out; a.y = static_cast<__nv_bfloat16*>(y);
     a.seq_start = seq_start; a.keep = nullptr;
     a.KH = k_heads; a.VH = v_heads; a.DV = dv; a.S = n_seqs;
-    void* args[] = {&a};
-    dim3 grid((dv + tf::kRowsPerCta - 1) / tf::kRowsPerCta, v_heads, n_seqs);
-    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<true>, grid, dim3(tf::kRowsPerCta * 2), 0,
-                                   static_cast<cudaStream_t>(stream), args);
+    const cudaError_t e = tf::launch_gdn<true>(a, n_seqs, stream);
     if (e != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
 }
@@ -524,10 +537,7 @@ int tf_gdn_replay(const void* k, const void* v, const float* g, const float* bet
     a.seq_start = seq_start; a.keep = keep;
     a.KH = k_heads; a.VH = v_heads; a.DV = dv; a.S = n_seqs;
     a.rec_q = rec_k_stride; a.rec_v = rec_v_stride; a.rec_g = rec_g_stride; a.rec_state = state_stride;
-    void* args[] = {&a};
-    dim3 grid((dv + tf::kRowsPerCta - 1) / tf::kRowsPerCta, v_heads, n_seqs * layers);
-    cudaError_t e = tf::launch_pdl((const void*)tf::gdn_kernel<false>, grid, dim3(tf::kRowsPerCta * 2), 0,
-                                   static_cast<cudaStream_t>(stream), args);
+    const cudaError_t e = tf::launch_gdn<false>(a, n_seqs * layers, stream);
     if (e != cudaSuccess) { cudaGetLastError(); return TF_ECUDA; }
     return TF_OK;
 }

@@ -57,3 +57,38 @@ def test_mixer_on_both_sides_of_a_block_an_sm(lib, widths, nk, nv, group):
     assert torch.equal(packed.data, want_packed.data)
     for got, want in zip(rec, (k, v, g, beta)):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("vh,windows,layers", [(4, 1, 1), (4, 6, 1), (4, 7, 1), (4, 9, 1), (4, 10, 1), (32, 1, 6), (32, 7, 1), (32, 1, 8)])
+def test_replay_has_the_chain_state_at_any_grid(lib, vh, windows, layers):
+    """Both sides of the lines between one and two value rows a thread, and between three and four blocks an SM."""
+
+    from tensorfold_b200 import lane_gdn
+
+    gen = torch.Generator(device="cuda").manual_seed(vh + windows)
+    width, kh = 3, vh // 2
+    rows = width * windows
+    rnd = lambda *s: torch.randn(s, generator=gen, device="cuda")
+    k = torch.nn.functional.normalize(rnd(layers, rows, kh, 128), dim=-1).to(torch.bfloat16)
+    v = rnd(layers, rows, vh, 128).to(torch.bfloat16)
+    g, beta = (torch.rand((layers, rows, vh), generator=gen, device="cuda") for _ in range(2))
+    state = 0.1 * rnd(layers, windows, vh, 128, 128)
+    starts = torch.arange(0, rows + 1, width, dtype=torch.int32, device="cuda")
+    want = torch.empty_like(state)
+    for i in range(layers):
+        for s in range(windows):                             # one window a call: the small grid
+            part = slice(s * width, (s + 1) * width)
+            final = torch.empty_like(state[i, s:s + 1])
+            y = lane_gdn.gated_delta_chain(k[i, part], k[i, part], v[i, part], g[i, part], beta[i, part], state[i, s:s + 1],
+                                           torch.tensor([0, width], dtype=torch.int32, device="cuda"), state_out=final)
+            want[i, s] = final[0]
+            if s == 0:
+                first = y
+        every = lane_gdn.gated_delta_chain(k[i], k[i], v[i], g[i], beta[i], state[i], starts)
+        assert_same_bits(every[:width], first, "chain rows")
+    keep = torch.full((windows,), width, dtype=torch.int32, device="cuda")
+    if layers == 1:
+        lane_gdn.replay(k[0], v[0], g[0], beta[0], state[0], starts, keep)
+    else:
+        lane_gdn.replay(k, v, g, beta, state, starts, keep)
+    assert_same_bits(state, want, "replayed states")
