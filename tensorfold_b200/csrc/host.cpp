@@ -6,7 +6,8 @@
 // of conversion for 17 arguments; tensors are passed as tensors), and the matmul calls do their checks,
 // allocations and launches in one native call.
 //
-// The functions take the arguments of the C entry point, in order: a pointer is a CUDA tensor, an address or None.
+// The functions take the arguments of the C entry point, in order: a pointer is a CUDA tensor, an address or None. While the
+// C call runs the interpreter is released, as under ctypes: a launch that waits for a place in a full queue stops no other thread.
 
 #include <Python.h>
 
@@ -28,6 +29,11 @@ namespace {
 std::atomic<long long> g_launches{0};      // kernels queued by successful calls
 
 struct PyErr {};                           // thrown with a Python error set
+
+struct Released {                          // the interpreter lock given up for a scope; no Python object is touched in it
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+};
 [[noreturn]] void fail(PyObject* type, const char* text) {
     PyErr_SetString(type, text);
     throw PyErr{};
@@ -72,10 +78,16 @@ struct Entry<Fn, LAUNCHES> {
     static PyObject* apply(PyObject* const* args, std::index_sequence<I...>) {
         std::tuple<A...> v{convert<A>(args[I])...};
         if constexpr (std::is_void_v<R>) {
-            Fn(std::get<I>(v)...);
+            {
+                const Released unlocked;
+                Fn(std::get<I>(v)...);
+            }
             Py_RETURN_NONE;
         } else {
-            const R rc = Fn(std::get<I>(v)...);
+            const R rc = [&] {
+                const Released unlocked;
+                return Fn(std::get<I>(v)...);
+            }();
             if (LAUNCHES > 0 && rc == 0) g_launches.fetch_add(LAUNCHES, std::memory_order_relaxed);
             return to_python(rc);
         }
@@ -182,8 +194,7 @@ PyObject* shaped(const at::Tensor& out, const at::Tensor& x, int64_t n) {
 // number, packed and multiplied in launches of up to TF_QMM_MAX_ROWS rows
 PyObject* lane_matmul_py(PyObject* const* args, Py_ssize_t) {
     at::AutoDispatchBelowADInplaceOrView no_grad;
-    const at::Tensor& x = tensor(args[0]);
-    const at::Tensor& w = tensor(args[1]);
+    const at::Tensor x = tensor(args[0]), w = tensor(args[1]);       // held: the interpreter lock is given up below
     const int n = convert<int>(args[2]), k = convert<int>(args[3]), group = convert<int>(args[4]);
     const bool f32 = convert<int>(args[5]) != 0;
     const at::Tensor x2 = rows_of(x, k, "lane_matmul", n);
@@ -198,25 +209,32 @@ PyObject* lane_matmul_py(PyObject* const* args, Py_ssize_t) {
     const int64_t most = m < TF_QMM_MAX_ROWS ? m : TF_QMM_MAX_ROWS;
     const at::Tensor packed = at::empty({(int64_t)tf_packed_bytes((int)most, k, group)}, x.options().dtype(at::kByte));
     const size_t out_row = (size_t)n * (f32 ? 4 : 2);
-    for (int64_t r0 = 0; r0 < m; r0 += TF_QMM_MAX_ROWS) {
-        const int rows = (int)std::min<int64_t>(m - r0, TF_QMM_MAX_ROWS);
-        const bool last = r0 + rows >= m;
-        check_rc(tf_pack_rows(static_cast<const uint8_t*>(x2.const_data_ptr()) + (size_t)r0 * k * 2, packed.mutable_data_ptr(), nullptr,
-                              rows, k, group, stream.stream()), "pack_rows");
-        check_rc(tf_qmm_next(packed.const_data_ptr(), w.const_data_ptr(), static_cast<uint8_t*>(out.mutable_data_ptr()) + r0 * out_row,
-                             scratch.mutable_data_ptr(), (size_t)scratch.numel(), rows, n, k, group, f32 ? TF_QMM_F32_OUT : 0,
-                             last ? next_w : w.const_data_ptr(), last ? next_n : n, last ? next_k : k, last ? next_group : group, status,
-                             stream.stream()), "lane_matmul");
-        g_launches.fetch_add(2, std::memory_order_relaxed);
-    }
+    const char* what = "pack_rows";
+    const int rc = [&] {
+        const Released unlocked;
+        for (int64_t r0 = 0; r0 < m; r0 += TF_QMM_MAX_ROWS) {
+            const int rows = (int)std::min<int64_t>(m - r0, TF_QMM_MAX_ROWS);
+            const bool last = r0 + rows >= m;
+            what = "pack_rows";
+            if (const int bad = tf_pack_rows(static_cast<const uint8_t*>(x2.const_data_ptr()) + (size_t)r0 * k * 2, packed.mutable_data_ptr(),
+                                             nullptr, rows, k, group, stream.stream())) return bad;
+            what = "lane_matmul";
+            if (const int bad = tf_qmm_next(packed.const_data_ptr(), w.const_data_ptr(), static_cast<uint8_t*>(out.mutable_data_ptr()) + r0 * out_row,
+                                            scratch.mutable_data_ptr(), (size_t)scratch.numel(), rows, n, k, group, f32 ? TF_QMM_F32_OUT : 0,
+                                            last ? next_w : w.const_data_ptr(), last ? next_n : n, last ? next_k : k,
+                                            last ? next_group : group, status, stream.stream())) return bad;
+            g_launches.fetch_add(2, std::memory_order_relaxed);
+        }
+        return (int)TF_OK;
+    }();
+    check_rc(rc, what);
     return shaped(out, x, n);
 }
 
 // prefill_matmul(x, tiled, n, k, group, f32, out, staging, status): the same on the wide-row kernel
 PyObject* prefill_matmul_py(PyObject* const* args, Py_ssize_t) {
     at::AutoDispatchBelowADInplaceOrView no_grad;
-    const at::Tensor& x = tensor(args[0]);
-    const at::Tensor& w = tensor(args[1]);
+    const at::Tensor x = tensor(args[0]), w = tensor(args[1]);       // held: the interpreter lock is given up below
     const int n = convert<int>(args[2]), k = convert<int>(args[3]), group = convert<int>(args[4]);
     const bool f32 = convert<int>(args[5]) != 0;
     const at::Tensor x2 = rows_of(x, k, "prefill_matmul", n);
@@ -231,15 +249,23 @@ PyObject* prefill_matmul_py(PyObject* const* args, Py_ssize_t) {
     if ((size_t)packed.numel() < need) fail(PyExc_ValueError, "prefill_matmul: staging buffer too small");
     int* status = convert<int*>(args[8]);
     const size_t out_row = (size_t)n * (f32 ? 4 : 2);
-    for (int64_t r0 = 0; r0 < m; r0 += TF_QMM_MAX_ROWS) {
-        const int rows = (int)std::min<int64_t>(m - r0, TF_QMM_MAX_ROWS);
-        check_rc(tf_pack_rows_tc(static_cast<const uint8_t*>(x2.const_data_ptr()) + (size_t)r0 * k * 2, packed.mutable_data_ptr(), nullptr,
-                                 rows, k, group, stream.stream()), "prefill pack_rows");
-        check_rc(tf_qmm_tc(packed.const_data_ptr(), w.const_data_ptr(), static_cast<uint8_t*>(out.mutable_data_ptr()) + r0 * out_row,
-                           scratch.mutable_data_ptr(), (size_t)scratch.numel(), rows, n, k, group, f32 ? TF_QMM_F32_OUT : 0, status,
-                           stream.stream()), "prefill_matmul");
-        g_launches.fetch_add(2, std::memory_order_relaxed);
-    }
+    const char* what = "prefill pack_rows";
+    const int rc = [&] {
+        const Released unlocked;
+        for (int64_t r0 = 0; r0 < m; r0 += TF_QMM_MAX_ROWS) {
+            const int rows = (int)std::min<int64_t>(m - r0, TF_QMM_MAX_ROWS);
+            what = "prefill pack_rows";
+            if (const int bad = tf_pack_rows_tc(static_cast<const uint8_t*>(x2.const_data_ptr()) + (size_t)r0 * k * 2, packed.mutable_data_ptr(),
+                                                nullptr, rows, k, group, stream.stream())) return bad;
+            what = "prefill_matmul";
+            if (const int bad = tf_qmm_tc(packed.const_data_ptr(), w.const_data_ptr(), static_cast<uint8_t*>(out.mutable_data_ptr()) + r0 * out_row,
+                                          scratch.mutable_data_ptr(), (size_t)scratch.numel(), rows, n, k, group, f32 ? TF_QMM_F32_OUT : 0,
+                                          status, stream.stream())) return bad;
+            g_launches.fetch_add(2, std::memory_order_relaxed);
+        }
+        return (int)TF_OK;
+    }();
+    check_rc(rc, what);
     return shaped(out, x, n);
 }
 
