@@ -127,7 +127,8 @@ def launch_count() -> int:
 
 class Bound:
     """The entry points as attributes: native functions that take the C arguments in order, a pointer being a CUDA
-    tensor, an address or None (``csrc/host.cpp``); ``cdll`` is the same library through ctypes."""
+    tensor, an address or None (``csrc/host.cpp``), or whatever else ctypes takes; ``cdll`` is the same library through
+    ctypes."""
 
 
 def load():
@@ -146,7 +147,7 @@ def load():
             fn = getattr(bound.cdll, name)
             fn.restype = res
             fn.argtypes = args
-            setattr(bound, name, getattr(host, name))
+            setattr(bound, name, host.bound(name, fn))
         _host, _lib = host, bound
     return _lib
 

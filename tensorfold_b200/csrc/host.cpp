@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <atomic>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -92,15 +93,21 @@ struct Entry<Fn, LAUNCHES> {
             return to_python(rc);
         }
     }
-    static PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t n) {
-        if (n != (Py_ssize_t)sizeof...(A)) {
-            PyErr_Format(PyExc_TypeError, "this entry point takes %d arguments, got %zd", (int)sizeof...(A), n);
-            return nullptr;
-        }
+    // `self` is the entry point through ctypes where bound() made the function: it takes what the conversions here do not
+    // (ctypes objects, byref, arrays, sizes to be wrapped), or says why not.
+    static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+        const bool bound = self != nullptr && PyCallable_Check(self);
         try {
-            return apply(args, std::index_sequence_for<A...>{});
+            if (n == (Py_ssize_t)sizeof...(A)) return apply(args, std::index_sequence_for<A...>{});
+            PyErr_Format(PyExc_TypeError, "this entry point takes %d arguments, got %zd", (int)sizeof...(A), n);
+            throw PyErr{};
         } catch (const PyErr&) {
-            return nullptr;
+            if (!bound || !(PyErr_ExceptionMatches(PyExc_TypeError) || PyErr_ExceptionMatches(PyExc_OverflowError))) return nullptr;
+            PyErr_Clear();
+            PyObject* result = PyObject_Vectorcall(self, args, (size_t)n, nullptr);
+            if (LAUNCHES > 0 && result != nullptr && PyLong_Check(result) && PyLong_AsLong(result) == 0)
+                g_launches.fetch_add(LAUNCHES, std::memory_order_relaxed);
+            return result;
         } catch (const std::exception& e) {
             PyErr_SetString(PyExc_RuntimeError, e.what());
             return nullptr;
@@ -277,6 +284,8 @@ PyObject* stream_py(PyObject* const* args, Py_ssize_t n) {
 PyObject* device_py(PyObject* const*, Py_ssize_t) { return PyLong_FromLong(c10::cuda::current_device()); }
 PyObject* count_py(PyObject* const*, Py_ssize_t) { return PyLong_FromLongLong(g_launches.load(std::memory_order_relaxed)); }
 
+PyObject* bound_py(PyObject* const* args, Py_ssize_t n);
+
 #define TF_FN(name, launches) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&Entry<&name, launches>::call)), METH_FASTCALL, nullptr}
 #define TF_OWN(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(&guarded<&fn>)), METH_FASTCALL, nullptr}
 
@@ -293,9 +302,18 @@ PyMethodDef methods[] = {
     TF_FN(tf_moe_combine_peer, 1), TF_FN(tf_moe_pack, 1), TF_FN(tf_moe_act, 1), TF_FN(tf_moe_combine, 1), TF_FN(tf_peer_slot_bytes, 0),
     TF_FN(tf_peer_exchange, 1), TF_FN(tf_qmm_act, 1), TF_FN(tf_swiglu_tiled, 1), TF_FN(tf_qmm_peer, 1), TF_FN(tf_norm_xs_peer, 1),
     TF_FN(tf_set_poll_limit, 0), TF_FN(tf_topk_scratch_bytes, 0), TF_FN(tf_topk_rows, 2), TF_FN(tf_topk_sample_rows, 2), TF_FN(tf_sample_rows, 1),
-    TF_OWN("scratch", scratch_py), TF_OWN("lane_matmul", lane_matmul_py), TF_OWN("prefill_matmul", prefill_matmul_py),
+    TF_OWN("bound", bound_py), TF_OWN("scratch", scratch_py), TF_OWN("lane_matmul", lane_matmul_py), TF_OWN("prefill_matmul", prefill_matmul_py),
     TF_OWN("current_stream", stream_py), TF_OWN("current_device", device_py), TF_OWN("launch_count", count_py),
     {nullptr, nullptr, 0, nullptr}};
+
+// bound(name, fn): the entry point `name`, with `fn` (the same one through ctypes) for the arguments it does not convert itself
+PyObject* bound_py(PyObject* const* args, Py_ssize_t n) {
+    const char* name = n == 2 ? PyUnicode_AsUTF8(args[0]) : nullptr;
+    if (name == nullptr) fail(PyExc_TypeError, "bound(name, function)");
+    for (PyMethodDef* def = methods; def->ml_name != nullptr; ++def)
+        if (std::strcmp(def->ml_name, name) == 0) return PyCFunction_NewEx(def, args[1], nullptr);
+    fail(PyExc_AttributeError, name);
+}
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native binding of libtensorfold_b200.so", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

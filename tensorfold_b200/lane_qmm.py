@@ -227,7 +227,7 @@ def lane_matmul(x: torch.Tensor | Packed, weight, scales: torch.Tensor | None = 
     if not isinstance(x, Packed):
         if peer is None and act_out is None:
             # plain rows: checks, allocations, packing and launches in one native call
-            return _lib.host().lane_matmul(x, weight.tiled, weight.n, weight.k, weight.group, f32, out, *hint,
+            return _lib.host().lane_matmul(x, weight.tiled, weight.n, weight.k, weight.group, bool(f32), out, *hint,
                                            _lib.status(x.device).word if x.is_cuda else None)
         if x.shape[-1] != weight.k:
             raise ValueError(f"lane_matmul: weight (N={weight.n}, K={weight.k}) does not match K={x.shape[-1]}")

@@ -69,7 +69,7 @@ def prefill_matmul(x, weight: TCWeight, *, f32: bool = False, out: torch.Tensor 
 
     if not isinstance(x, Packed):
         # plain rows: checks, allocations, packing and launches in one native call
-        return _lib.host().prefill_matmul(x, weight.tiled, weight.n, weight.k, weight.group, f32, out, staging,
+        return _lib.host().prefill_matmul(x, weight.tiled, weight.n, weight.k, weight.group, bool(f32), out, staging,
                                           _lib.status(x.device).word if x.is_cuda else None)
     lib = _lib.load()
     if x.k != weight.k or x.group != weight.group:

@@ -68,3 +68,25 @@ def test_product_has_no_oracle_or_cpu_path():
     for path in pkg.rglob("*.py"):
         text = path.read_text()
         assert "oracle" not in text.replace("no CPU or PyTorch fallback", ""), path
+
+
+def test_entry_points_take_what_ctypes_takes(lib):
+    """The native functions convert tensors, addresses and None themselves; any other argument ctypes accepts still goes through."""
+
+    from tensorfold_b200 import _lib
+
+    buf = (ctypes.c_char * 4096)()
+    p = (ctypes.addressof(buf) + 255) & ~255
+    v, i = ctypes.c_void_p, ctypes.c_int
+    assert lib.tf_packed_bytes(i(8), i(5120), 64) == lib.tf_packed_bytes(8, 5120, 64) > 0
+    assert lib.tf_qmm(v(p), v(p), v(p), v(None), ctypes.c_size_t(1 << 30), i(8), 64, 64, 64, 0, v(None), None) == _lib.TF_ESCRATCH
+    assert lib.tf_qmm(buf, p, ctypes.byref(buf, 256), None, 1 << 30, 0, 64, 64, 64, 0, None, None) == _lib.TF_EINVAL
+    assert lib.tf_qmm(p, p, p, p, -1, 0, 64, 64, 64, 0, None, None) == _lib.TF_EINVAL          # a size that wraps, as in C
+    before = _lib.launch_count()
+    for bad in ((1.5, 64, 64), (8, "64", 64), (8, 64)):
+        try:
+            lib.tf_packed_bytes(*bad)
+        except (TypeError, ctypes.ArgumentError):
+            continue
+        raise AssertionError(f"{bad} was taken")
+    assert _lib.launch_count() == before

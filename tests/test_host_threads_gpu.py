@@ -41,3 +41,18 @@ def test_a_full_queue_stops_no_other_thread(lib, call):
     torch.cuda.synchronize()
     assert took[0] > 0.5, "the queue was never full: the test shows nothing"
     assert longest < 0.3, f"this thread stood still for {longest:.2f} s"
+
+
+def test_f32_is_a_truth_value(lib):
+    """Any object with a truth value, as before the checks went into native code."""
+
+    import numpy as np
+
+    from tensorfold_b200 import lane_qmm, prefill_qmm, synthetic
+
+    x = torch.randn((2, 128), device="cuda").to(torch.bfloat16)
+    w = synthetic.random_q4(torch.Generator(device="cuda").manual_seed(1), 256, 128, 64, "cuda")
+    wide = prefill_qmm.tile_weight(*lane_qmm.untile_weight(w), 64)
+    for yes, no in ((np.True_, np.False_), ("yes", ""), ([1], None)):
+        for call, q in ((lane_qmm.lane_matmul, w), (prefill_qmm.prefill_matmul, wide)):
+            assert call(x, q, f32=yes).dtype == torch.float32 and call(x, q, f32=no).dtype == torch.bfloat16
