@@ -3,7 +3,8 @@
 ``python -m tensorfold_b200.build`` compiles every ``csrc/*.cu`` with nvcc into
 ``tensorfold_b200/libtensorfold_b200.so`` next to this file. The library is plain C ABI
 (``include/tensorfold_b200.h``) and needs only nvcc; ``csrc/host.cpp``, the native Python binding that takes
-torch tensors, is compiled with g++ into ``_host.so`` beside it and linked against it.
+torch tensors, is compiled with g++ against the headers of this Python and this torch into ``_host.so`` beside it and linked
+against it. The Python package needs both.
 """
 
 from __future__ import annotations
@@ -28,6 +29,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--fmad=false",
 ]
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-w"]
 
 
 def _nvcc() -> str:
@@ -48,20 +50,34 @@ def source_hash() -> str:
     return h.hexdigest()
 
 
-def _build_host(force: bool) -> None:
-    """``csrc/host.cpp`` -> ``_host.so``: rebuilt when it, the C header or the torch it is compiled against changed."""
+def host_digest() -> str:
+    """What ``_host.so`` is made from: its source and the C header, the compiler flags, and the Python and torch it is compiled against."""
 
     import sysconfig
 
     import torch
 
-    src, header = CSRC / "host.cpp", HERE.parent / "include" / "tensorfold_b200.h"
-    digest = hashlib.sha256(src.read_bytes() + header.read_bytes() + torch.__version__.encode()).hexdigest()
+    h = hashlib.sha256()
+    for path in (CSRC / "host.cpp", HERE.parent / "include" / "tensorfold_b200.h"):
+        h.update(path.read_bytes())
+    made_for = [*HOST_FLAGS, sys.version, str(sysconfig.get_config_var("SOABI")), torch.__version__, str(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    h.update("\0".join(made_for).encode())
+    return h.hexdigest()
+
+
+def _build_host(force: bool) -> None:
+    """``csrc/host.cpp`` -> ``_host.so``, where ``host_digest`` says that it would differ."""
+
+    import sysconfig
+
+    import torch
+
+    src, digest = CSRC / "host.cpp", host_digest()
     if not force and HOST.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text().strip() == digest:
         return
     t = Path(torch.__file__).parent
     cuda = Path(_nvcc()).resolve().parent.parent
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+    cmd = ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            f"-I{sysconfig.get_paths()['include']}", f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{cuda}/include", str(src),
            "-o", str(HOST), f"-L{HERE}", "-ltensorfold_b200", f"-L{t}/lib", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
            "-Wl,-rpath,$ORIGIN"]
