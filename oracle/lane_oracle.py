@@ -18,12 +18,7 @@ kernels against themselves (row alone == row in a window), never against this fi
 
 from __future__ import annotations
 
-import os
 from dataclasses import dataclass, field
-
-# one BLAS code path on every x86 host: the pinned outputs were made on another CPU model, and some models' default
-# fp32 summation order moves single bf16 roundings, which the recurrence carries on to the following rows
-os.environ.setdefault("MKL_CBWR", "COMPATIBLE")
 
 import numpy as np
 import torch

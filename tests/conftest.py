@@ -1,5 +1,11 @@
+import os
 import sys
 from pathlib import Path
+
+# One BLAS code path on every x86 host, set before torch is first imported: the oracle's pinned outputs were made on another
+# CPU model, and some models' default fp32 summation order moves single bf16 roundings, which the recurrence carries on to
+# the following rows. Here and not in the oracle, which the benchmark times: it takes MKL two to five times longer.
+os.environ.setdefault("MKL_CBWR", "COMPATIBLE")
 
 import pytest
 

@@ -13,8 +13,11 @@ generators, so a test can rebuild the same inputs from the seed and compare outp
 
 from __future__ import annotations
 
+import os
 import sys
 from pathlib import Path
+
+os.environ.setdefault("MKL_CBWR", "COMPATIBLE")      # as the tests that compare with these files (tests/conftest.py)
 
 import numpy as np
 import torch
