@@ -69,9 +69,10 @@ def _tokens(rows: Sequence[int], device) -> torch.Tensor:
     return torch.tensor(list(rows), dtype=torch.int32, device=device)
 
 
-# Rows a prompt is processed in at a time where the caller does not say: every pass streams all weights, so the fewer
-# passes the better (203 tokens through 8 layers of the 27B-class model: 27.6 ms in passes of 8 rows), and a row's bits do not
-# depend on its companions.
+# Rows of a prompt that ``Engine`` processes at a time unless its ``prompt_rows`` says otherwise: every pass streams all weights,
+# so the fewer passes the better (203 tokens through 8 layers of the 27B-class model: 8.6 ms, 27.6 in passes of 8 rows), and a
+# row's bits do not depend on its companions. A pass's buffers grow with its rows, above all attention's partials: 24 heads of 256 at
+# 32768 keys take 355 MB for 128 rows, 22 MB for 8. (``prefill`` has its own ``chunk``, 8 rows a sequence unless given.)
 PROMPT_ROWS = MAX_ROWS
 
 
@@ -214,9 +215,13 @@ class Engine:
     exact stream: prefill through the lane forward, then drafted rounds (n-gram copy drafter) whose output is
     token for token what serial decoding gives. A prompt that extends the previous request's reuses its
     committed state (``State.snapshot`` / ``restore`` at the end of the shared prefix is the caller's tool for
-    anything finer)."""
+    anything finer). ``prompt_rows``: rows of a prompt processed in one pass, fewer where memory is short."""
 
-    def __init__(self, w: Weights, *, max_context: int = 8192, eos: Sequence[int] = (), max_rows: int = 8):
+    def __init__(self, w: Weights, *, max_context: int = 8192, eos: Sequence[int] = (), max_rows: int = 8,
+                 prompt_rows: int = PROMPT_ROWS):
+        if not 1 <= prompt_rows <= MAX_ROWS:
+            raise ValueError(f"1 <= prompt_rows <= {MAX_ROWS} required")
+        self.prompt_rows = prompt_rows
         self.w, self.eos, self.max_rows, self.max_context = w, tuple(int(t) for t in eos), max_rows, max_context
         self.state = State(w, 1, max_context)
         self.committed: list = []              # tokens whose state is committed
@@ -237,7 +242,7 @@ class Engine:
             keep = 0
         start = time.perf_counter()
         # a shared prefix is committed already: only the new tail runs; positions continue from it
-        pending = _prefill(self.w, self.state, [prompt[keep:]], sampling, PROMPT_ROWS, [len(prompt)])[0]
+        pending = _prefill(self.w, self.state, [prompt[keep:]], sampling, self.prompt_rows, [len(prompt)])[0]
         self.committed = list(prompt)
         out = [int(pending)]
         stopped = bool(on_tokens(list(out))) if on_tokens else False
