@@ -4,7 +4,7 @@ Mirror of the reference's ``engine/exact_sampling.py`` (``Sampling``, ``uniform_
 ``sample_rows``, ``MARGIN``) and of its CUDA ``sample_rows`` (``families/qwen3_5/cuda/sampling.py:13-34``).
 The token at absolute position p is the argmax over the kept candidates of ``logit/T + Gumbel(hash(seed,
 p, id))``: it depends only on the row's own logits and position, so a window row draws the token the
-serial step at that position draws. Candidates come from the GPU radix top-k; the draw runs on the
+serial step at that position draws. Candidates come from the GPU top-k; the draw runs on the
 GPU too (``tf_sample_rows``); ``choose_rows`` takes candidates in any order (merged vocabulary shards of a
 tensor-parallel head) and draws with the same kernel; there is no host-side draw in this package.
 """
@@ -33,7 +33,7 @@ class Sampling:
 
 def choose_rows(values, ids, positions: Sequence[int], s: Sampling) -> list[int]:
     """The draw for rows of candidate (value, id) pairs in any order (reference:
-    ``exact_sampling.choose_rows``), run on the GPU: the candidates are put in the order the radix top-k
+    ``exact_sampling.choose_rows``), run on the GPU: the candidates are put in the order the top-k
     writes them, (value descending, id ascending), and handed to the keyed draw kernel."""
 
     dev = torch.device("cuda")
@@ -78,7 +78,7 @@ def sample_rows(logits: torch.Tensor, positions, s: Sampling | None, *, top: tup
     if s is None or s.temperature <= 0:
         return topk_rows(logits, 1)[0].reshape(rows)
     if not 0 < int(s.top_k) <= MAX_K - MARGIN:
-        raise ValueError(f"sample_rows: top_k must be in 1..{MAX_K - MARGIN} (the radix top-k holds {MAX_K} candidates)")
+        raise ValueError(f"sample_rows: top_k must be in 1..{MAX_K - MARGIN} (the top-k kernel holds {MAX_K} candidates)")
     if not torch.is_tensor(positions):
         positions = torch.tensor(list(positions), dtype=torch.int64)
     positions = positions.to(device=logits.device, dtype=torch.int64)

@@ -179,20 +179,6 @@ def scratch_for(device: torch.device) -> torch.Tensor:
     return _lib.host().scratch(device.index or 0)
 
 
-_tiled_cache: dict[tuple, QWeight] = {}
-
-
-def _as_qweight(weight, scales, biases) -> QWeight:
-    """The reference's call shape: stored words + scales + biases. Tiled once per (words, scales, biases)
-    storage and remembered, as the reference remembers its regrouped weights."""
-
-    key = (weight.data_ptr(), scales.data_ptr(), biases.data_ptr(), tuple(weight.shape))
-    q = _tiled_cache.get(key)
-    if q is None:
-        q = _tiled_cache[key] = tile_weight(weight, scales, biases)
-    return q
-
-
 def lane_matmul(x: torch.Tensor | Packed, weight, scales: torch.Tensor | None = None, biases: torch.Tensor | None = None, *,
                 xs: torch.Tensor | None = None, sk: int | None = None, f32: bool = False,
                 out: torch.Tensor | None = None, next_weight: QWeight | None = None, peer=None,
@@ -202,7 +188,7 @@ def lane_matmul(x: torch.Tensor | Packed, weight, scales: torch.Tensor | None = 
 
     ``weight`` is a ``QWeight`` (tiled once by ``tile_weight``) or, in the reference's call shape
     ``lane_matmul(x, weight, scales, biases, xs=..., sk=...)``, the stored (N, K/8) words with their scales
-    and biases (tiled on first use). ``xs`` (the input's group sums) is accepted for that call shape and not
+    and biases (tiled in the call, for that call: tile once with ``tile_weight`` to keep it). ``xs`` (the input's group sums) is accepted for that call shape and not
     needed: packing forms the sums; ``sk`` must be None or the shape's own ``split_k``.
     ``f32``: return the unrounded fp32 sums (a tensor-parallel rank's partial). More than
     ``MAX_ROWS`` rows run as several launches; a row's bits do not depend on which launch it rides in.
@@ -219,7 +205,7 @@ def lane_matmul(x: torch.Tensor | Packed, weight, scales: torch.Tensor | None = 
     if not isinstance(weight, QWeight):
         if scales is None or biases is None:
             raise ValueError("lane_matmul: stored words need their scales and biases")
-        weight = _as_qweight(weight, scales, biases)
+        weight = tile_weight(weight, scales, biases)
     if sk is not None and sk != split_k(weight.n, weight.k):
         raise ValueError(f"lane_matmul: the K schedule is fixed by the shape (split_k = {split_k(weight.n, weight.k)}), got sk={sk}")
     nw = next_weight

@@ -1,8 +1,9 @@
-"""Top-k over vocabulary rows, exact and deterministic: radix select on bf16 keys.
+"""Top-k over vocabulary rows, exact and deterministic, on sortable bf16 keys.
 
 Mirror of the reference's ``engine/topk.py:130-146`` (``topk_rows``): value descending, ties to the
-lower token id, k <= ``MAX_K``. A row is cut into slices (one CTA each) whose candidates a second
-kernel ranks; a row's result depends on that row alone.
+lower token id, k <= ``MAX_K``. A row is cut into slices (one CTA each), each slice's
+candidates, those that reach a lower bound of its k-th largest key, are ranked there, and a second kernel
+ranks the slices' lists; a row's result depends on that row alone.
 """
 
 from __future__ import annotations

@@ -40,3 +40,25 @@ def test_a_weight_refilled_in_place_is_the_one_read(lib, rows, n, k):
     fresh = lane_qmm.tile_weight(*raw, 64)                  # the tiling kernel right in front
     assert_same_bits(lane_qmm.lane_matmul(x, fresh), want_b, "just tiled")
     assert_same_bits(lane_qmm.lane_matmul(x, *raw), want_b, "tiled inside the call")
+
+
+@pytest.mark.gpu
+def test_stored_weights_are_read_at_every_call(lib):
+    """The call shape with stored words: other values at the same addresses, however they got there, are the ones multiplied."""
+
+    from tensorfold_b200 import lane_qmm
+
+    gen = torch.Generator().manual_seed(3)
+    a, b = (O.random_q4(gen, 300, 128, 64) for _ in range(2))
+    x = torch.randn((3, 128), generator=gen).to(torch.bfloat16).cuda()
+    cuda = lambda q: [t.cuda() for t in (q.words, q.scales, q.biases)]
+    want = [lane_qmm.lane_matmul(x, lane_qmm.tile_weight(*cuda(q), 64)) for q in (a, b)]
+    held = cuda(a)
+    assert_same_bits(lane_qmm.lane_matmul(x, *held), want[0], "first values")
+    for t, new in zip(held, cuda(b)):
+        t.data.copy_(new)
+    assert_same_bits(lane_qmm.lane_matmul(x, *held), want[1], "overwritten in place")
+    for i in (0, 1, 0, 1):                                   # freed and allocated again, at the same addresses
+        del held
+        held = cuda((a, b)[i])
+        assert_same_bits(lane_qmm.lane_matmul(x, *held), want[i], "new tensors")
