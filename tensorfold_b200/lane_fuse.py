@@ -39,7 +39,8 @@ class _Group:
     added: int              # bytes the stack holds beyond its members (tile padding)
 
 
-_stacks: dict[int, dict[str, _Group]] = {}
+# id(layer) -> (layer, its stacks): the layer is held until ``clear``, so that no other object can come to its id
+_stacks: dict[int, tuple[dict, dict[str, _Group]]] = {}
 
 
 def _stack(layer: dict, kind: str, device, group: int) -> _Group:
@@ -60,7 +61,7 @@ def build(model: dict, device="cuda") -> dict[str, int]:
     for layer in model["layers"]:
         for kind, names in GROUPS.items():
             if all(name in layer for name in names):
-                _stacks.setdefault(id(layer), {})[kind] = _stack(layer, kind, device, group)
+                _stacks.setdefault(id(layer), (layer, {}))[1][kind] = _stack(layer, kind, device, group)
                 counts[kind] += 1
     return counts
 
@@ -78,14 +79,14 @@ def stats(model: dict) -> dict:
     counts = {kind: 0 for kind in GROUPS}
     added = 0
     for layer in model["layers"]:
-        for kind, g in _stacks.get(id(layer), {}).items():
+        for kind, g in _stacks.get(id(layer), (layer, {}))[1].items():
             counts[kind] += 1
             added += g.added
     return {"groups": counts, "added_bytes": added}
 
 
 def _project(layer: dict, kind: str, x):
-    g = _stacks.get(id(layer), {}).get(kind)
+    g = _stacks.get(id(layer), (layer, {}))[1].get(kind)
     if g is None:
         return None
     if not isinstance(x, Packed) and x.dtype != torch.bfloat16:
