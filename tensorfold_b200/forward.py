@@ -96,6 +96,7 @@ class Weights:
     head: QWeight
     inv_freq: torch.Tensor
     wide: dict | None = None          # id(QWeight) -> prefill_qmm.TCWeight, made by enable_wide
+    wide_of: list | None = None       # the QWeights of ``wide``, held so that no other one can come to their ids
 
     def nbytes(self) -> int:
         """Bytes of 4-bit projection weights one forward streams (the weight-bytes roofline numerator)."""
@@ -125,6 +126,7 @@ def enable_wide(w: Weights) -> Weights:
         for q in mats:
             words, scales, biases = untile_weight(q)
             w.wide[id(q)] = prefill_qmm.tile_weight(words, scales, biases, q.group)
+        w.wide_of = mats
     return w
 
 

@@ -95,3 +95,18 @@ def test_prompt_rows_bound_the_memory_of_a_pass(weights):
     for bad in (0, 129):
         with pytest.raises(ValueError):
             decode.Engine(weights, max_context=512, prompt_rows=bad)
+
+
+def test_a_replaced_weight_has_no_wide_twin(lib):
+    """The wide twins belong to the weights they were made from: another weight in their place is not given one silently."""
+
+    import weakref
+
+    from tensorfold_b200 import forward as F, synthetic
+
+    w = F.enable_wide(F.load_weights(O.random_model(O.Config(**DENSE), seed=45), "cuda"))
+    old = weakref.ref(w.head)
+    w.head = synthetic.random_q4(torch.Generator(device="cuda").manual_seed(1), w.head.n, w.head.k, w.head.group, "cuda")
+    assert old() is not None
+    with pytest.raises(KeyError):
+        F.tree_forward(w, torch.zeros(1, dtype=torch.int32, device="cuda"), [1], F.State(w, 1, 64, wide=True))
